@@ -65,6 +65,8 @@ struct Prog {
 // per strip.)
 constexpr unsigned kSlotAll = 0xffffffffu;  // cleared count: every column
 
+struct WalkBall;
+
 struct PairDesc {
   const double* P;        // curve 1, [n1][d]
   const double* Q;        // curve 2, [n2][d]
@@ -88,6 +90,10 @@ struct PairDesc {
   // the pair's grid (n1 then counts the mirror's rows + 1).  0 for every other descriptor.
   int split, mrow;
   long long cstride, tstride;
+  // walk groups (rfd_walk.cuh): bounds of the shorter curve's chunks, records per block row of
+  // the longer curve (null: the pair is walked by one CTA)
+  const struct WalkBall* balls;
+  void* recs;
 };
 
 struct PairState {
@@ -117,6 +123,9 @@ struct PairState {
   int kary_left;  // the pair: decisions of the round still running
   int kary_in;    // this decision belongs to a round
   int kary_reach; // its outcome
+  int walk_off;   // the walk gave the pair up: the strips take it
+  int walk_band;  // the pair's records say where a walk's band ran
+  double walk_ve; // VE-FD result a walk found ahead of the DFD (0: none)
   int corner;     // mirror decision: the far corner lies in the free space (see split_sync_kernel)
 };
 
@@ -415,6 +424,7 @@ __device__ __forceinline__ unsigned bcast(unsigned v) { return __shfl_sync(kFull
 __device__ __forceinline__ unsigned long long bcast(unsigned long long v) {
   return __shfl_sync(kFull, v, 0);
 }
+__device__ __forceinline__ double bcast_f64(double v) { return __shfl_sync(kFull, v, 0); }
 
 struct Waiter {
   long long t0, budget;

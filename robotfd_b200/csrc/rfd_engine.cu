@@ -29,6 +29,7 @@
 #include "rfd_dfd.cuh"
 #include "rfd_filter.h"
 #include "rfd_team.cuh"
+#include "rfd_walk.cuh"
 #include "rfd_features.cuh"
 #include "rfd_mlp.h"
 
@@ -211,11 +212,11 @@ __global__ void __launch_bounds__(kBlock) wave_kernel(WaveArgs wa) {
 // again, now coupled to the next anchor; on a diagonal step prefixes pair with prefixes, then
 // suffixes with suffixes.  Every full pair then lies within |a - b| + inflation(a) +
 // inflation(b) of a coupled anchor pair (a, b), so the DFD of the anchors with those cell
-// weights, squared, is at least the DFD of the curves.  One block per pair (grid-stride);
+// weights, squared, is at least the DFD of the curves.  Grid as prep_kernel;
 // pairs with coarse = 0 keep the DFD.
 __global__ void coarse_prep_kernel(const PairDesc* pairs, const PairDesc* coarse, PairState* st,
                                    int npairs, int k) {
-  for (int p = blockIdx.x; p < npairs; p += gridDim.x) {
+  for (int p = blockIdx.y; p < npairs; p += gridDim.y) {
     // a pair with a one-point curve (coarse = 0): every point, inflation 0, so the inflated
     // sweep computes its exact DFD
     const bool exact = !st[p].coarse;
@@ -249,7 +250,8 @@ __global__ void coarse_prep_kernel(const PairDesc* pairs, const PairDesc* coarse
       };
       // each anchor: its coordinates and its inflation (each block's radii are computed by
       // its own two anchors: no thread reads another's result)
-      for (long long a = threadIdx.x; a < cn; a += blockDim.x) {
+      for (long long a = blockIdx.x * blockDim.x + threadIdx.x; a < cn;
+           a += (long long)gridDim.x * blockDim.x) {
         const long long at = anchor(a);
         for (int e = 0; e < d; ++e) Y[a * ds + e] = X[at * d + e];
         const double before = !exact && a > 0 ? block_radius(a - 1, true) : 0.0;
@@ -756,6 +758,275 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) team_kernel(WaveArgs
   }
 }
 
+// ---- walk sweeps (rfd_walk.cuh)
+
+// Pairs of a launch, longest first, and the CTAs that share one (plan[0] pairs, plan[1] CTAs,
+// plan[2..] the pairs).
+struct WalkArgs {
+  const int* plan;
+  unsigned* ticket;
+  int phases;              // 1 DFD, 2 VE-FD, 4 search
+  int quota;               // probes per pair in this launch
+  // groups: arrival counts and announced pairs by group, reports and ends by CTA
+  unsigned* arrive;
+  int* next;               // [2][grid]
+  WalkStat* stats;         // [2][grid]
+  WalkEnd* ends;           // [3][grid]
+};
+
+// Root mean square length of up to 32 segments of a curve (stride: doubles per point).
+__device__ __forceinline__ double sample_spacing_sq(const double* X, int n, int d) {
+  const int lane = threadIdx.x & 31;
+  double s = 0.0;
+  if (n >= 2) {
+    const double* a = X + (size_t)((long long)(n - 1) * lane / 32) * d;
+    for (int k = 0; k < d; ++k) s += (a[d + k] - a[k]) * (a[d + k] - a[k]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+  return s / 32.0;
+}
+
+// The reference's launch rule of the VE-FD (finalize): int product of the point counts.
+__device__ __forceinline__ bool walk_skips_vefd(int quirks, const PairDesc& pd) {
+  return quirks && (int)((unsigned)pd.n1 * (unsigned)pd.n2) <= 10000;
+}
+
+// The phases of one pair, one after another, as far as the walk takes them, by the CTAs of a
+// group together: every member comes to the same results, the first one keeps the pair's state.
+// Returns false on an error (the error word is set).
+__device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh, Walk& w,
+                          WalkGroup& g, int p) {
+  const int lane = threadIdx.x & 31;
+  PairState* st = wa.st + p;
+  const bool leader = g.rank == 0;
+  auto geti = [&](const int* x) { return bcast(lane == 0 ? ld_volatile(x) : 0); };
+  auto getd = [&](const double* x) { return bcast_f64(lane == 0 ? *(const volatile double*)x : 0.0); };
+  __syncwarp();
+  if (lane == 0) {
+    PairDesc d = wa.pairs[p];
+    if (d.n1 < d.n2) {  // rows along the longer curve
+      const double* t = d.P;
+      d.P = d.Q;
+      d.Q = t;
+      const int n = d.n1;
+      d.n1 = d.n2;
+      d.n2 = n;
+      d.tr ^= 1;
+    }
+    sh->pd = d;
+    sh->filter = st->filter;
+    sh->mat = st->formula == 1;
+  }
+  __syncwarp();
+  w.cut0 = w.cut1 = -1;
+  w.near_lo = 0;
+  w.near_hi = -1;
+  const bool pieces = g.size > 1 && sh->pd.recs;
+  // Rounds beyond the first two that a phase may take in all: a quarter of what the strips need
+  // for it (DFD 0.25 us a point, the others 7 us a strip or 3 us a chunk) at 10 us a round and
+  // 6 us a block row of a piece.
+  const double long_us = 3.0 / 32.0 * sh->pd.n1, round_us = 10.0 + 6.0 / 32.0 * sh->pd.n1 / g.size;
+  const int limit_dfd = 8 + (int)(0.25 * 0.25 * (sh->pd.n1 + sh->pd.n2) / round_us);
+  const int limit_dec = 8 + (int)(0.25 * fmax(long_us, 7.0 / 32.0 * sh->pd.n2) / round_us);
+  // Where an earlier launch's sweep found the band, pieces start from it.
+  bool band = pieces && geti(&st->walk_band) != 0;
+  if (band) {
+    const int nbr = (sh->pd.n1 + 30) >> 5, nbc = (sh->pd.n2 + 30) >> 5;
+    const int np = walk_pieces(sh->pd, g.size, nbr, nbc);
+    if (np > 1 && g.rank < np)
+      walk_cut(w, (const WalkRecord*)sh->pd.recs, nbr, nbc, np, g.rank);
+    if (!walk_barrier(wa, g)) return false;  // (before a record changes)
+  }
+  // a radius to grow a level from: the larger of the endpoint bound and f x the points' spacing
+  auto first_radius = [&](double f) {
+    const double s = sqrt(fmax(sample_spacing_sq(sh->pd.P, sh->pd.n1, sh->pd.d),
+                               sample_spacing_sq(sh->pd.Q, sh->pd.n2, sh->pd.d)));
+    return fmax(fmax(getd(&st->endpoint), f * s), 1e-100);
+  };
+  for (int probes = 0;;) {
+    const int phase = geti(&st->phase);
+    if (!geti(&st->active) || geti(&st->walk_off)) return true;
+    double res = 0.0;
+    int rc = WALK_OK;
+    if (phase == PH_DFD && (ka.phases & 1)) {
+      // No upper bound is at hand: sweep at a level that grows fourfold (radii twofold) until a
+      // path survives.  A surviving sweep's result is exact; one that dies ends where its band
+      // does.
+      //
+      // A group does the VE-FD first: its level can be so low that the band is a cell or two wide
+      // and every piece meets its record at once, and the DFD's pieces then start near that band.
+      w.rounds = 0;
+      double rad = first_radius(1.0);
+      if (pieces && !walk_skips_vefd(geti(&st->quirks), sh->pd)) {
+        double r = first_radius(0.5);
+        for (int it = 0; it < 64; ++it, r *= 2.0) {
+          const double level = __dmul_rn(r, r);
+          rc = walk_value<K_VEFD>(wa, sh, w, g, level, getd(&st->seed), limit_dec, band, res);
+          if (rc != WALK_OK || res <= level) break;
+        }
+        if (rc == WALK_OK && res < kFltMax) {
+          if (leader && lane == 0) st->walk_ve = res;
+          rad = fmax(rad, sqrt(res));
+        }
+        if (rc == WALK_ERROR) return false;
+        if (rc == WALK_GIVE_UP && !walk_barrier(wa, g)) return false;
+      }
+      w.rounds = 0;
+      for (int it = 0;; ++it, rad *= 2.0) {
+        rc = it == 64 ? WALK_GIVE_UP
+                      : walk_value<K_DFD>(wa, sh, w, g, __dmul_rn(rad, rad), 0.0, limit_dfd, band,
+                                          res);
+        if (rc != WALK_OK || res < kFltMax) break;
+      }
+      if (rc == WALK_OK && leader && lane == 0) {
+        st->result = res;
+        finalize<K_DFD>(st, wa.pairs[p], wa.active_pairs);
+      }
+    } else if (phase == PH_VEFD && (ka.phases & 2)) {
+      const double U = getd(&st->U), seed = getd(&st->seed);
+      const double ve = getd(&st->walk_ve);  // found ahead of the DFD
+      // The exact DFD leaves a band that one CTA walks in the same time as a thinner one; a
+      // coarse bound may leave most of the grid, and a group's pieces meet their records the
+      // sooner the thinner the band is, so there the level grows up to the bound.
+      const bool grow = geti(&st->coarse) != 0 || pieces;
+      double rad = grow ? first_radius(0.5) : 0.0;
+      w.rounds = 0;
+      for (;; rad *= 2.0) {
+        if (ve > 0.0) {
+          res = ve <= U ? ve : kFltMax;
+          break;
+        }
+        const double level = grow ? fmin(__dmul_rn(rad, rad), U) : U;
+        rc = walk_value<K_VEFD>(wa, sh, w, g, level, seed, limit_dec, band, res);
+        if (rc != WALK_OK || res <= level || !(level < U)) break;
+      }
+      if (lane == 0 && sh->cells) atomicAdd(&st->cells_vefd, sh->cells);
+      if (rc == WALK_OK && leader && lane == 0) {
+        st->result = res;
+        finalize<K_VEFD>(st, wa.pairs[p], wa.active_pairs);
+      }
+    } else if (phase == PH_SEARCH && (ka.phases & 4) && probes < ka.quota) {
+      ++probes;
+      w.rounds = 0;
+      WalkSweep o{false, INT_MAX, limit_dec, 0.0, false, false};
+      rc = walk_sweep<K_DEC>(wa, sh, w, g, getd(&st->r2), getd(&st->split), 0.0, o, res);
+      if (lane == 0 && sh->cells) {
+        atomicAdd(&st->cells_eval, sh->cells);
+        atomicAdd(&st->cells_fp64, sh->cells64 / 2);
+      }
+      if (rc == WALK_OK && leader && lane == 0) {
+        st->result = res;
+        finalize<K_DEC>(st, wa.pairs[p], wa.active_pairs);
+      }
+    } else {
+      return true;
+    }
+    __syncwarp();
+    if (lane == 0) {
+      sh->cells = sh->cells64 = 0ull;
+      if (rc == WALK_GIVE_UP && leader) st->walk_off = 1;
+      if (leader && band) st->walk_band = 1;
+    }
+    if (rc == WALK_ERROR || !walk_barrier(wa, g)) return false;
+  }
+}
+
+// One pair at a time per group of CTAs (one CTA, or several co-resident ones: a cooperative
+// launch), longest pairs first.  What the walk gives up stays in its phase for the strips.
+__global__ void __launch_bounds__(kWalkThreads, 2) walk_kernel(WaveArgs wa, WalkArgs ka) {
+  extern __shared__ __align__(128) unsigned char team_smem[];
+  WalkShared* sh = (WalkShared*)team_smem;
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 2; ++k) {
+      mbar_init(&sh->full[k], kWalkHelpers);
+      mbar_init(&sh->req[k], 1);
+    }
+    sh->cells = sh->cells64 = 0ull;
+  }
+  __syncthreads();
+  const int n = __ldg(ka.plan), size = __ldg(ka.plan + 1);
+  const int grid = gridDim.x, group = blockIdx.x / size;
+  if ((group + 1) * size > grid || group >= n) return;
+  if (threadIdx.x >= 32) {
+    walk_helpers(wa, sh);
+    return;
+  }
+  const int lane = threadIdx.x;
+  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, 0, -1, -1, -1, 0, -1, 0};
+  WalkGroup g;
+  g.size = size;
+  g.rank = blockIdx.x - group * size;
+  g.first = group * size;
+  g.passed = 0;
+  g.arrive = ka.arrive + group;
+  for (int k = 0; k < 2; ++k) g.stat[k] = ka.stats + (size_t)k * grid;
+  for (int k = 0; k < 3; ++k) g.end[k] = ka.ends + (size_t)k * grid;
+  for (int turn = 0;; ++turn) {
+    // the group's next pair: taken by its first member
+    int t = 0;
+    if (g.rank == 0 && lane == 0) {
+      t = ld_volatile(wa.error) ? INT_MAX : (int)min(atomicAdd(ka.ticket, 1u), 0x7fffffffu);
+      if (size > 1) __stcg(ka.next + (size_t)(turn & 1) * grid + group, t);
+    }
+    if (size > 1) {
+      if (!walk_barrier(wa, g)) break;
+      if (lane == 0) t = __ldcg(ka.next + (size_t)(turn & 1) * grid + group);
+    }
+    t = bcast(t);
+    if (t >= n || !walk_pair(wa, ka, sh, w, g, __ldg(ka.plan + 2 + t))) break;
+  }
+  walk_request(sh, w, kStop, 0);
+}
+
+// The pairs still in the phase, in order, and the CTAs each can have (1 .. most): plan.
+__global__ void __launch_bounds__(1024) walk_plan_kernel(const int* order, const PairState* st,
+                                                         int npairs, int phase, int grid, int most,
+                                                         int* plan) {
+  __shared__ int warp_n[32];
+  __shared__ int base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) base = 0;
+  __syncthreads();
+  for (int k0 = 0; k0 < npairs; k0 += 1024) {
+    const int k = k0 + threadIdx.x;
+    const int p = k < npairs ? order[k] : 0;
+    const bool in = k < npairs && st[p].active && st[p].phase == phase && !st[p].walk_off;
+    const unsigned b = __ballot_sync(kFull, in);
+    if (lane == 0) warp_n[warp] = __popc(b);
+    __syncthreads();
+    int at = base;
+    for (int q = 0; q < warp; ++q) at += warp_n[q];
+    if (in) plan[2 + at + __popc(b & ((1u << lane) - 1u))] = p;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int q = 0; q < 32; ++q) base += warp_n[q];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    plan[0] = base;
+    plan[1] = max(1, min(most, grid / max(base, 1)));
+  }
+}
+
+// Bounds of the shorter curve's chunks of every pair that has room for them.
+__global__ void walk_ball_kernel(const PairDesc* pairs, int npairs) {
+  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int warps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int p = blockIdx.y; p < npairs; p += gridDim.y) {
+    const PairDesc d = pairs[p];
+    if (!d.balls) continue;
+    const bool swap = d.n1 < d.n2;
+    const double* X = swap ? d.P : d.Q;
+    const int n = swap ? d.n1 : d.n2;
+    WalkBall* out = const_cast<WalkBall*>(d.balls);
+    for (int j = warp; j < (n + 31) / 32; j += warps) {
+      if (d.d == 2) walk_ball<2>(X, n, j, out + j);
+      else walk_ball<3>(X, n, j, out + j);
+    }
+  }
+}
+
 // ---- meet in the middle (one pair's VE-FD and search decisions)
 //
 // A split pair's forward sweep runs its first k strips (grid rows 0 .. 32k - 1) and its mirror
@@ -936,21 +1207,22 @@ __global__ void __launch_bounds__(kFeatThreads) features_kernel(const PairDesc* 
   }
 }
 
-// Per-pair constants and state.  One block per pair (grid-stride).
+// Per-pair constants and state.  Pairs over grid rows (y), a pair's segments over grid columns.
 __global__ void prep_kernel(const PairDesc* pairs, PairState* st, int npairs, int start_phase) {
-  for (int p = blockIdx.x; p < npairs; p += gridDim.x) {
+  const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (int p = blockIdx.y; p < npairs; p += gridDim.y) {
     const PairDesc pd = pairs[p];
     const int d = pd.d;
     double2* rowc = const_cast<double2*>(pd.rowc);
     double2* colrec = const_cast<double2*>(pd.colrec);
-    for (int i = threadIdx.x; i < pd.n1 - 1; i += blockDim.x) {
+    for (int i = first; i < pd.n1 - 1; i += stride) {
       double t[3] = {0.0, 0.0, 0.0};
       for (int k = 0; k < d; ++k)
         t[k] = __dsub_rn(pd.P[(size_t)(i + 1) * d + k], pd.P[(size_t)i * d + k]);
       const double A = d == 3 ? sq_sum<3>(t) : sq_sum<2>(t);
       rowc[i] = make_double2(A, __ddiv_rn(0.5, A));
     }
-    for (int j = threadIdx.x; j < pd.n2 - 1; j += blockDim.x) {
+    for (int j = first; j < pd.n2 - 1; j += stride) {
       double q0[3] = {0, 0, 0}, q1[3] = {0, 0, 0}, t[3] = {0, 0, 0};
       for (int k = 0; k < d; ++k) {
         q0[k] = pd.Q[(size_t)j * d + k];
@@ -972,7 +1244,7 @@ __global__ void prep_kernel(const PairDesc* pairs, PairState* st, int npairs, in
         r[3] = make_double2(A, inv);
       }
     }
-    if (threadIdx.x == 0) {
+    if (first == 0) {
       PairState* s = st + p;
       // endpoint bound: host arithmetic in the reference, no fusion (src/frechet.cpp:30)
       double a = 0.0, b = 0.0;
@@ -1025,6 +1297,9 @@ struct rfd_context {
   int team_grid[3] = {0, 0, 0};     // teams of the chosen shape (team_warps)
   int team_grids[2][3] = {{0, 0, 0}, {0, 0, 0}};  // [teams of 4, of 8 warps][kind]
   int team_warps = 8;  // warps per team: 8 or 4 (RFD_TEAM_WARPS, rfd_autotune_search)
+  // walk sweeps first (rfd_walk.cuh), the strips for what they give up; RFD_WALK=0: strips only
+  int walk = 1;
+  int walk_grid = 0;
   int solo = 0;  // RFD_SOLO=1: VE-FD and decisions on the solo-warp strips (A/B checks)
   int lockstep = 0;  // RFD_LOCKSTEP=1: one launch per probe round instead of the continuous search
   int search_switch = 0;  // active pairs below which the continuous search takes over
@@ -1063,6 +1338,13 @@ struct rfd_context {
 namespace {
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+// Grid of prep_kernel and coarse_prep_kernel: a block per 1024 points of the longest curve
+// (about 2000 blocks in all) by the pairs.
+dim3 prep_grid(int64_t longest, int64_t npairs) {
+  const int64_t gx = std::max<int64_t>(1, std::min<int64_t>((longest + 1023) / 1024, 256));
+  return dim3((unsigned)gx, (unsigned)std::min<int64_t>(npairs, std::max<int64_t>(1, 2048 / gx)));
+}
 
 // The team kernel of the context's shape (warps per team) on its grid (grid > 0: that many
 // teams); MIR: the mirror kernel of split pairs.
@@ -1479,6 +1761,15 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   L.ntitems = (int)ntitems;
   L.items = take(sizeof(int2) * nitems);
   L.titems = take(sizeof(int2) * ntitems);
+  // walk: pairs longest first, plans (host-made for the first launches, device-made for the
+  // search's tail), the groups' words
+  const bool walks = ctx->walk && !o.dense && !ctx->solo && !ctx->prof;
+  const size_t order_off = take(sizeof(int) * npairs);
+  const size_t plan_off = take(sizeof(int) * (2 + npairs) * 3);
+  const int64_t wg = walks ? ctx->walk_grid : 0;
+  const size_t wnext_off = take(sizeof(int) * 2 * wg);
+  const size_t wstat_off = take(sizeof(WalkStat) * 2 * wg);
+  const size_t wend_off = take(sizeof(WalkEnd) * 3 * wg);
   L.tdescs = take(sizeof(PairDesc) * nst);
   L.states = take(sizeof(PairState) * nst);
   // ticket counters: DFD, two VE-FD, probe rounds (+1 for a decision), the continuous
@@ -1491,6 +1782,9 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   const int64_t wtickets =
       (nsplit ? (twin ? 2 * nwin : 1) : nwin) * (2 + std::max(max_probes, 1));
   L.zero_begin = off;
+  // the walk's ticket counters and groups' arrival counts, a set per launch
+  constexpr int kWalkLaunches = 8;
+  const size_t walk_ticket = take(sizeof(unsigned) * kWalkLaunches * (1 + wg));
   L.counters = take(sizeof(unsigned) * (wbase + wtickets));
   const size_t prof_off = take(sizeof(unsigned long long) * (kTraceBase + kTraceW * kTrace));
   L.error = take(sizeof(int));
@@ -1556,6 +1850,30 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       cQ[p] = take(sizeof(double) * (full ? n2 : coarse_n(n2)) * (d + 1));
     }
   }
+  // walk groups: chunk bounds of the shorter curve and a record per block row of the longer one
+  // (about 34 bytes a point), longest pairs first, within kWalkBytes in all; a pair without
+  // them is walked by one CTA
+  // A pair with one long curve, kWalkAspect times the other's length, stays on the strips: rows along
+  // the shorter curve make them few, and a spacing far below the distance a band that is wide
+  // along the denser curve.
+  constexpr int kWalkAspect = 8, kWalkAspectFrom = 8192;
+  constexpr size_t kWalkBytes = (size_t)1 << 30;
+  std::vector<size_t> wball(npairs, 0), wrec(npairs, 0);
+  std::vector<int> worder(npairs);
+  for (int64_t p = 0; p < npairs; ++p) worder[p] = (int)p;
+  std::stable_sort(worder.begin(), worder.end(),
+                   [&](int a, int b) { return n1s[a] + n2s[a] > n1s[b] + n2s[b]; });
+  if (walks) {
+    const size_t w0 = off;
+    for (int64_t k = 0; k < npairs; ++k) {
+      const int p = worder[k];
+      const int64_t lo = std::min(n1s[p], n2s[p]), hi = std::max(n1s[p], n2s[p]);
+      if (off - w0 + sizeof(WalkRecord) * ((hi + 31) / 32) > kWalkBytes && npairs > 1) break;
+      if (lo < 2) continue;
+      wrec[p] = take(sizeof(WalkRecord) * ((hi + 31) / 32));
+      wball[p] = take(sizeof(WalkBall) * ((lo + 31) / 32));
+    }
+  }
   for (int64_t v = 0; v < nmem; ++v) {
     const int64_t p = mpair(v);
     const int64_t St = (std::max<int64_t>(trows(p) - 1, 0) + 31) / 32;
@@ -1571,6 +1889,8 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   L.h_states = htake(sizeof(PairState) * nst);
   L.h_items = htake(sizeof(int2) * nitems);
   L.h_titems = htake(sizeof(int2) * ntitems);
+  const size_t h_order = htake(sizeof(int) * npairs);
+  const size_t h_plan = htake(sizeof(int) * (2 + npairs) * 2);
   L.h_misc = htake(4 * sizeof(int));
   const size_t h_src = dcompact ? htake(sizeof(SrcCurve) * 2 * npairs) : 0;
   L.h_curves = hoff;
@@ -1622,6 +1942,8 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     D.tags = (unsigned*)(dbase + L.tags[p]);
     D.prog = (Prog*)(dbase + L.prog[p]);
     D.slots = (unsigned long long*)(dbase + L.slots[p]);
+    D.balls = wball[p] ? (const WalkBall*)(dbase + wball[p]) : nullptr;
+    D.recs = wrec[p] ? dbase + wrec[p] : nullptr;
     D.ring = L.ring_d[p];
     D.n1 = (int)n1;
     D.n2 = (int)n2;
@@ -1686,6 +2008,8 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     s.blo = s.bhi = NAN;
     s.coarse = (ck && n1 >= 2 && n2 >= 2) ? 1 : 0;
     s.formula = formula[p];
+    s.walk_off = walks && std::max(n1, n2) >= kWalkAspectFrom &&
+                 std::max(n1, n2) >= kWalkAspect * std::min(n1, n2);
     if (o.bracket && mode == MODE_DISTANCE) {
       s.blo = o.bracket[2 * p];
       s.bhi = o.bracket[2 * p + 1];
@@ -1778,6 +2102,35 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     if (twin && !nsplit) wstart[nwin] = (int)k;
   }
 
+  // Walk plans.  With pairs for less than half the CTAs each pair gets a group of its own, the
+  // CTAs shared out evenly.  Otherwise the pairs that alone would take longer than twice an
+  // even share of all blocks go first, in groups, and the others one CTA each.
+  int wsize[2] = {1, 1};   // CTAs per group of the two plans
+  int64_t wcount[2] = {0, 0};
+  if (walks) {
+    int* ho = (int*)(hbase + h_order);
+    int* hp = (int*)(hbase + h_plan);
+    for (int64_t p = 0; p < npairs; ++p) ho[p] = worder[p];
+    auto len = [&](int64_t k) { return (n1s[worder[k]] + n2s[worder[k]]) / 32 + 2; };
+    auto rows = [&](int64_t k) { return (std::max(n1s[worder[k]], n2s[worder[k]]) + 31) / 32; };
+    double all = 0.0;
+    for (int64_t k = 0; k < npairs; ++k) all += (double)len(k);
+    int64_t lead = npairs;
+    if (2 * npairs > wg) {
+      lead = 0;
+      while (lead < npairs && (double)len(lead) > std::max(64.0, 2.0 * all / (double)wg)) ++lead;
+    }
+    if (lead) wsize[0] = (int)std::max<int64_t>(1, std::min(wg / lead, rows(0) / 2));
+    wcount[0] = lead;
+    wcount[1] = npairs - lead;
+    for (int s = 0; s < 2; ++s) {
+      int* q = hp + (size_t)s * (2 + npairs);
+      q[0] = (int)wcount[s];
+      q[1] = wsize[s];
+      for (int64_t k = 0; k < wcount[s]; ++k) q[2 + k] = worder[(s ? lead : 0) + k];
+    }
+  }
+
   if (!on_device) {
     // Copy every curve into the pinned staging area (compacting repeated points with
     // drop_repeats).  Large batches split the pairs over host threads by bytes: a single
@@ -1842,13 +2195,30 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   // as one CUDA graph; a later call with the same layout (sizes, options, workspace) replays it,
   // reading the new inputs from the same pinned staging area.
   int launches = 0;
+  bool capturing = false;
   // Phase events.  Inside a stream capture a plain record only orders the capture; an
   // external record becomes a graph node, so the replayed graph records the events.
   auto record = [&](int k) {
     return cudaEventRecordWithFlags(ctx->ev[k], st,
-                                    o.graph ? cudaEventRecordExternal : cudaEventRecordDefault);
+                                    capturing ? cudaEventRecordExternal : cudaEventRecordDefault);
   };
-  auto issue = [&]() -> int {
+  const PairDesc* dd = (const PairDesc*)(dbase + L.descs);
+  const PairDesc* dt = (const PairDesc*)(dbase + L.tdescs);  // team strips' orientation
+  PairState* ds = (PairState*)(dbase + L.states);
+  WaveArgs wa{};
+  wa.pairs = dt;
+  wa.st = ds;
+  wa.items = (const int2*)(dbase + L.titems);
+  wa.nitems = L.ntitems;
+  wa.error = (int*)(dbase + L.error);
+  wa.active_pairs = (int*)(dbase + L.active);
+  wa.spin_cycles = ctx->spin_cycles;
+  wa.prof = ctx->prof ? (unsigned long long*)(dbase + prof_off) : nullptr;
+  int64_t longest = 1;
+  for (int64_t p = 0; p < npairs; ++p) longest = std::max({longest, n1s[p], n2s[p]});
+
+  // Inputs to the device, per-pair constants and states.
+  auto upload = [&]() -> int {
     RFD_CUDA(cudaMemcpyAsync(dbase + L.descs, hbase + L.h_descs, sizeof(PairDesc) * npairs,
                              cudaMemcpyHostToDevice, st));
     if (ck) {
@@ -1864,6 +2234,12 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
                              cudaMemcpyHostToDevice, st));
     RFD_CUDA(cudaMemcpyAsync(dbase + L.titems, hbase + L.h_titems, sizeof(int2) * ntitems,
                              cudaMemcpyHostToDevice, st));
+    if (walks) {
+      RFD_CUDA(cudaMemcpyAsync(dbase + order_off, hbase + h_order, sizeof(int) * npairs,
+                               cudaMemcpyHostToDevice, st));
+      RFD_CUDA(cudaMemcpyAsync(dbase + plan_off, hbase + h_plan, sizeof(int) * (2 + npairs) * 2,
+                               cudaMemcpyHostToDevice, st));
+    }
     if (dcompact) {
       // the caller's curves (pointers refreshed every call) compacted into the workspace
       RFD_CUDA(cudaMemcpyAsync(dbase + src_off, hbase + h_src, sizeof(SrcCurve) * 2 * npairs,
@@ -1882,25 +2258,97 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     RFD_CUDA(cudaMemsetAsync(dbase + L.zero_begin, 0, L.zero_end - L.zero_begin, st));
     RFD_CUDA(cudaMemcpyAsync(dbase + L.active, hmisc, sizeof(int), cudaMemcpyHostToDevice, st));
 
-    // ---------------- launches
-    const PairDesc* dd = (const PairDesc*)(dbase + L.descs);
-    const PairDesc* dt = (const PairDesc*)(dbase + L.tdescs);  // team strips' orientation
-    PairState* ds = (PairState*)(dbase + L.states);
     const int start_phase = mode == MODE_DECIDE ? PH_SEARCH : PH_DFD;
     if (ctx->timing) RFD_CUDA(record(0));
     launches = 1;
-    prep_kernel<<<(int)std::min<int64_t>(npairs, 8 * ctx->num_sms), 256, 0, st>>>(dt, ds, (int)npairs,
-                                                                                  start_phase);
+    prep_kernel<<<prep_grid(longest, npairs), 256, 0, st>>>(dt, ds, (int)npairs, start_phase);
     RFD_CUDA(cudaGetLastError());
-    WaveArgs wa{};
-    wa.pairs = dt;
-    wa.st = ds;
-    wa.items = (const int2*)(dbase + L.titems);
-    wa.nitems = L.ntitems;
-    wa.error = (int*)(dbase + L.error);
-    wa.active_pairs = (int*)(dbase + L.active);
-    wa.spin_cycles = ctx->spin_cycles;
-    wa.prof = ctx->prof ? (unsigned long long*)(dbase + prof_off) : nullptr;
+    if (ck) {
+      coarse_prep_kernel<<<prep_grid((longest + ck - 1) / ck, npairs), 256, 0, st>>>(
+          dd, (const PairDesc*)(dbase + cdescs), ds, (int)npairs, ck);
+      RFD_CUDA(cudaGetLastError());
+      ++launches;
+    }
+    if (walks && wsize[0] > 1) {
+      walk_ball_kernel<<<prep_grid(longest, npairs), 256, 0, st>>>(dt, (int)npairs);
+      RFD_CUDA(cudaGetLastError());
+      ++launches;
+    }
+    return RFD_OK;
+  };
+
+  // The learned bracket of every pair waiting for it.
+  auto network = [&]() -> int {
+    rfd_model* md = const_cast<rfd_model*>(o.model);
+    if (rfd_mlp::model_device(md) != ctx->device)
+      return fail(RFD_ERR_ARG, "the model lives on another device");
+    float* feat = (float*)(dbase + feat_off);
+    float* yout = (float*)(dbase + y_off);
+    bracket_features_kernel<<<(int)std::min<int64_t>(npairs, 16 * ctx->num_sms), kFeatThreads, 0,
+                              st>>>(dd, ds, (int)npairs, feat);
+    RFD_CUDA(cudaGetLastError());
+    int rc2 = rfd_mlp::infer(md, feat, (int)npairs, yout, st);
+    if (rc2) return rc2;
+    bracket_apply_kernel<<<(int)std::min<int64_t>((npairs + 255) / 256, 1024), 256, 0, st>>>(
+        ds, (int)npairs, yout, wa.active_pairs);
+    RFD_CUDA(cudaGetLastError());
+    launches += 2 + 4;
+    return RFD_OK;
+  };
+
+  // Walk sweeps of the phases in `phases` (WalkArgs) of a plan's pairs, one launch; groups need
+  // its CTAs co-resident.  Plan 2 is made on the device.
+  int nwalk = 0;
+  auto walk_launch = [&](int plan, bool groups, int64_t ctas, int phases, int quota) -> int {
+    WalkArgs ka{};
+    ka.plan = (const int*)(dbase + plan_off) + (size_t)plan * (2 + npairs);
+    ka.ticket = (unsigned*)(dbase + walk_ticket) + (size_t)nwalk * (1 + wg);
+    ka.arrive = ka.ticket + 1;
+    ka.phases = phases;
+    ka.quota = quota;
+    ka.next = (int*)(dbase + wnext_off);
+    ka.stats = (WalkStat*)(dbase + wstat_off);
+    ka.ends = (WalkEnd*)(dbase + wend_off);
+    ++nwalk;
+    const int g = (int)std::min<int64_t>(ctas, wg);
+    if (groups) {
+      void* args[] = {&wa, &ka};
+      RFD_CUDA(cudaLaunchCooperativeKernel((const void*)walk_kernel, dim3(g), dim3(kWalkThreads),
+                                           args, kWalkSmem, st));
+    } else {
+      walk_kernel<<<g, kWalkThreads, kWalkSmem, st>>>(wa, ka);
+      RFD_CUDA(cudaGetLastError());
+    }
+    ++launches;
+    return RFD_OK;
+  };
+  auto walk_plans = [&](int phases, int quota) -> int {
+    for (int s = 0; s < 2; ++s) {
+      if (!wcount[s]) continue;
+      const int rc = walk_launch(s, wsize[s] > 1, wcount[s] * wsize[s], phases, quota);
+      if (rc) return rc;
+    }
+    return RFD_OK;
+  };
+  // The phases in `phases`.  Where the pairs outnumber the CTAs a search starts with
+  // kWalkFirst probes of every pair; the few that need more then share the CTAs, twice.
+  constexpr int kWalkFirst = 2, kWalkSecond = 8;
+  auto walk = [&](int phases) -> int {
+    const bool tail = (phases & 4) && mode == MODE_DISTANCE && wcount[1] > 0;
+    int rc = walk_plans(phases, tail ? kWalkFirst : INT_MAX);
+    for (int k = 0; k < 2 && tail && !rc; ++k) {
+      walk_plan_kernel<<<1, 1024, 0, st>>>((const int*)(dbase + order_off), ds, (int)npairs,
+                                           PH_SEARCH, (int)wg, 32,
+                                           (int*)(dbase + plan_off) + 2 * (2 + npairs));
+      RFD_CUDA(cudaGetLastError());
+      ++launches;
+      rc = walk_launch(2, true, wg, 4, k ? INT_MAX : kWalkSecond);
+    }
+    return rc;
+  };
+
+  // The phases on strips, those in `parts`: 1 DFD, 2 VE-FD (and the bracket), 4 search.
+  auto strips = [&](int parts) -> int {
     unsigned* counters = (unsigned*)(dbase + L.counters);
     int li = 0;
     // boundary rows of the pairs about to run `ph` back to "not yet written" (team strips)
@@ -1985,16 +2433,11 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       launches += (int)(2 * nwin - 1);  // the caller counts one team launch
       return RFD_OK;
     };
-    if (mode != MODE_DECIDE) {
+    if (parts & 1) {
       wa.phase = PH_DFD;
       wa.ticket = counters + li++;
       // the DFD sweep runs on the coarse pairs when the coarse upper bound is asked for
       const PairDesc* ddfd = ck ? (const PairDesc*)(dbase + cdescs) : dd;
-      if (ck) {
-        coarse_prep_kernel<<<(int)std::min<int64_t>(npairs, 8 * ctx->num_sms), 256, 0, st>>>(
-            dd, ddfd, ds, (int)npairs, ck);
-        ++launches;
-      }
       // The coarse pair has k times fewer points per curve: one row per lane gives its sweep
       // the most strips in flight (long pair, k = 6: 21 ms against 38 with four rows).
       const int rows = ck ? 1 : ctx->dfd_rows;
@@ -2037,6 +2480,9 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       wa.nitems = L.ntitems;
       RFD_CUDA(cudaGetLastError());
       if (ctx->timing) RFD_CUDA(record(1));
+    }
+    li = 1;
+    if (parts & 2) {
       for (int ph : {PH_VEFD, PH_VEFD_DENSE}) {
         wa.phase = ph;
         wa.ticket = counters + li++;
@@ -2050,22 +2496,12 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       }
       launches += 3;
       if (use_model) {
-        rfd_model* md = const_cast<rfd_model*>(o.model);
-        if (rfd_mlp::model_device(md) != ctx->device)
-          return fail(RFD_ERR_ARG, "the model lives on another device");
-        float* feat = (float*)(dbase + feat_off);
-        float* yout = (float*)(dbase + y_off);
-        bracket_features_kernel<<<(int)std::min<int64_t>(npairs, 16 * ctx->num_sms), kFeatThreads, 0,
-                                  st>>>(dd, ds, (int)npairs, feat);
-        RFD_CUDA(cudaGetLastError());
-        int rc2 = rfd_mlp::infer(md, feat, (int)npairs, yout, st);
-        if (rc2) return rc2;
-        bracket_apply_kernel<<<(int)std::min<int64_t>((npairs + 255) / 256, 1024), 256, 0, st>>>(
-            ds, (int)npairs, yout, wa.active_pairs);
-        RFD_CUDA(cudaGetLastError());
-        launches += 2 + 4;
+        const int rc = network();
+        if (rc) return rc;
       }
     }
+    li = 3;
+    if (!(parts & 4)) return RFD_OK;
     if (ctx->timing) RFD_CUDA(record(2));
     const int nprobe = mode == MODE_DECIDE ? 1 : max_probes;
     wa.kary_k = karity;
@@ -2126,11 +2562,62 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       ++launches;
     }
     if (ctx->timing) RFD_CUDA(record(3));
+    return RFD_OK;
+  };
 
-    // ---------------- results
+  auto read_back = [&]() -> int {
     RFD_CUDA(cudaMemcpyAsync(hs, ds, sizeof(PairState) * npairs, cudaMemcpyDeviceToHost, st));
     RFD_CUDA(cudaMemcpyAsync(hmisc + 1, wa.error, sizeof(int), cudaMemcpyDeviceToHost, st));
     return RFD_OK;
+  };
+
+  // Walk sweeps first, unless every cell is asked for or the strips' own switches are set; the
+  // search of a call with k-ary members runs on the strips.  With phase timing each phase is a
+  // launch of its own.
+  auto issue = [&]() -> int {
+    int rc = upload();
+    if (rc) return rc;
+    if (!walks) {
+      rc = strips(mode == MODE_DECIDE ? 4 : 7);
+      return rc ? rc : read_back();
+    }
+    nwalk = 0;
+    const int search = nmem == 0 ? 4 : 0;
+    // The DFD stays on the strips with the coarse bound, whose level opens most of the coarse
+    // grid, and where the pairs outnumber the CTAs: the strips then run at the FP64 rate
+    // (5e11 cells/s), and the walk's few sweeps take as long.
+    const int dfd = ck || wcount[1] > 0 ? 0 : 1;
+    if (!dfd && mode != MODE_DECIDE) {
+      rc = strips(1);
+      if (rc) return rc;
+    }
+    if (mode == MODE_DECIDE) {
+      rc = walk(4);
+    } else if (!search) {
+      // (the strips also take what the walk gave up: the continuous search ends with the last
+      // active pair, so every pair has to come to it)
+      rc = walk(2 | dfd);
+      if (!rc) rc = strips(7);
+      return rc ? rc : read_back();
+    } else if (ctx->timing) {
+      if (dfd) rc = walk(1);
+      if (rc) return rc;
+      RFD_CUDA(record(1));
+      rc = walk(2);
+      if (!rc && use_model) rc = network();
+      if (rc) return rc;
+      RFD_CUDA(record(2));
+      rc = walk(4);
+    } else if (use_model) {
+      rc = walk(2 | dfd);
+      if (!rc) rc = network();
+      if (!rc) rc = walk(4);
+    } else {
+      rc = walk(2 | dfd | search);
+    }
+    if (rc) return rc;
+    if (ctx->timing) RFD_CUDA(record(3));
+    return read_back();
   };
   const bool use_graph = o.graph != 0;
   uint64_t key = 1469598103934665603ull;  // FNV-1a over everything the launches depend on
@@ -2145,7 +2632,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
                          ctx->search_switch, ctx->search_window, ctx->team_warps,
                          (int)(ctx->spin_cycles >> 32),
                          (int)(ctx->spin_cycles & 0xffffffff), karity, kary_gate, (int)twin,
-                         (int)nsplit, ctx->split_min};
+                         (int)nsplit, ctx->split_min, (int)walks};
     const void* ptrs[] = {dbase, hbase, gmodel, gmodel ? rfd_mlp::buffers_id(gmodel) : nullptr,
                           (const void*)st};
     mix(flags, sizeof(flags));
@@ -2166,8 +2653,10 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
       ctx->gexec = nullptr;
       RFD_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+      capturing = true;
     }
     const int rc = issue();
+    capturing = false;
     if (use_graph) {
       cudaGraph_t g = nullptr;
       const cudaError_t ec = cudaStreamEndCapture(st, &g);
@@ -2191,6 +2680,20 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     }
   }
   RFD_CUDA(cudaStreamSynchronize(st));
+  if (walks && hmisc[1] == 0) {
+    // what the walk gave up, from the phase it was in (bit 1 << phase), on the strips
+    unsigned open = 0;
+    for (int64_t p = 0; p < npairs; ++p)
+      if (hs[p].phase != PH_DONE) open |= 1u << hs[p].phase;
+    if (open) {
+      const int parts = ((open >> PH_DFD) & 1) | (open & ~(1u << PH_SEARCH) ? 2 : 0) | 4;
+      RFD_CUDA(cudaMemsetAsync(dbase + L.zero_begin, 0, L.zero_end - L.zero_begin, st));
+      int rc2 = strips(parts);
+      if (!rc2) rc2 = read_back();
+      if (rc2) return rc2;
+      RFD_CUDA(cudaStreamSynchronize(st));
+    }
+  }
   if (guard) {
     std::vector<unsigned char> g(guard);
     RFD_CUDA(cudaMemcpy(g.data(), dbase + L.total, guard, cudaMemcpyDeviceToHost));
@@ -2400,6 +2903,17 @@ int32_t rfd_context_create(int32_t device, rfd_context** out) {
       delete c;
       return fail(RFD_ERR_CUDA, "cudaFuncSetAttribute(team smem)");
     }
+    const char* wk = getenv("RFD_WALK");
+    c->walk = !(wk && wk[0] == '0');
+    int ow = 0;
+    if (cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kWalkSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ow, walk_kernel, kWalkThreads, kWalkSmem) !=
+            cudaSuccess) {
+      delete c;
+      return fail(RFD_ERR_CUDA, "cudaFuncSetAttribute(walk smem)");
+    }
+    c->walk_grid = std::max(1, ow) * c->num_sms;
     int o[4] = {0, 0, 0, 0};
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o[0], team_kernel<K_VEFD, 4>, 128, sm_ve);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o[1], team_kernel<K_DEC, 4>, 128, sm_dec);
@@ -2956,7 +3470,8 @@ std::mutex g_noalloc_mu;
 NoAllocDevice g_noalloc[64];
 
 __global__ void noalloc_setup_kernel(PairDesc* desc, PairState* st, int2* items, int nitems,
-                                     int* active, PairDesc d, double radius, double r2) {
+                                     int* active, int* order, PairDesc d, double radius,
+                                     double r2) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t == 0) {
     *desc = d;
@@ -2970,6 +3485,8 @@ __global__ void noalloc_setup_kernel(PairDesc* desc, PairState* st, int2* items,
     s.blo = s.bhi = CUDART_NAN;
     *st = s;
     *active = 1;
+    order[0] = order[1] = 1;  // one pair, one CTA
+    order[2] = 0;
   }
   for (int k = t; k < nitems; k += gridDim.x * blockDim.x) items[k] = make_int2(0, k);
 }
@@ -3012,6 +3529,8 @@ extern "C" int32_t rfd_decide_noalloc(const double* c1, int64_t n1, const double
       RFD_CUDA(cudaDeviceGetAttribute(&clk, cudaDevAttrClockRate, dev));
       nd.scratch = (unsigned char*)p;
       nd.team_grid = std::max(1, occ) * nsm;
+      RFD_CUDA(cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kWalkSmem));
       nd.spin_cycles = (long long)clk * 1000LL * 20LL;
       nd.ready = 1;
     }
@@ -3030,10 +3549,12 @@ extern "C" int32_t rfd_decide_noalloc(const double* c1, int64_t n1, const double
   const size_t o_zero = off;
   const size_t o_ticket = take(sizeof(unsigned));
   const size_t o_error = take(sizeof(int));
+  const size_t o_walk = o_ticket + 64;  // (inside the same 256 bytes)
   const size_t o_tags = take(sizeof(unsigned) * (size_t)ring * tstride);
   const size_t o_prog = take(sizeof(Prog) * S);
   const size_t zero_end = off;
   const size_t o_active = take(sizeof(int));
+  const size_t o_order = o_active + 64;  // (inside the same 256 bytes)
   const size_t o_rowc = take(sizeof(double2) * (size_t)(n1 - 1));
   const size_t o_colrec = take(sizeof(double2) * (dims == 2 ? 3 : 4) * (size_t)(n2 - 1));
   const size_t o_bnd = take(sizeof(double) * (size_t)ring * cstride);
@@ -3062,12 +3583,10 @@ extern "C" int32_t rfd_decide_noalloc(const double* c1, int64_t n1, const double
   PairState* dstate = (PairState*)(base + o_state);
   RFD_CUDA(cudaMemsetAsync(base + o_zero, 0, zero_end - o_zero, st));
   noalloc_setup_kernel<<<(int)std::min<int64_t>((S + 255) / 256, 64) + 1, 256, 0, st>>>(
-      ddesc, dstate, (int2*)(base + o_items), (int)S, (int*)(base + o_active), d, radius,
-      radius * radius);
+      ddesc, dstate, (int2*)(base + o_items), (int)S, (int*)(base + o_active),
+      (int*)(base + o_order), d, radius, radius * radius);
   RFD_CUDA(cudaGetLastError());
-  prep_kernel<<<1, 256, 0, st>>>(ddesc, dstate, 1, PH_SEARCH);
-  RFD_CUDA(cudaGetLastError());
-  bnd_fill_kernel<<<dim3(256, 1), 256, 0, st>>>(ddesc, dstate, 1, PH_SEARCH, nullptr, nullptr, 0);
+  prep_kernel<<<prep_grid(std::max(n1, n2), 1), 256, 0, st>>>(ddesc, dstate, 1, PH_SEARCH);
   RFD_CUDA(cudaGetLastError());
   WaveArgs wa{};
   wa.pairs = ddesc;
@@ -3080,6 +3599,16 @@ extern "C" int32_t rfd_decide_noalloc(const double* c1, int64_t n1, const double
   wa.active_pairs = (int*)(base + o_active);
   wa.spin_cycles = env_spin_cycles(nd.spin_cycles);
   wa.prof = nullptr;
+  // the walk, then the strips, whose launches end at once when the walk has decided
+  WalkArgs ka{};
+  ka.plan = (const int*)(base + o_order);
+  ka.ticket = (unsigned*)(base + o_walk);
+  ka.phases = 4;
+  ka.quota = 1;
+  walk_kernel<<<1, kWalkThreads, kWalkSmem, st>>>(wa, ka);
+  RFD_CUDA(cudaGetLastError());
+  bnd_fill_kernel<<<dim3(256, 1), 256, 0, st>>>(ddesc, dstate, 1, PH_SEARCH, nullptr, nullptr, 0);
+  RFD_CUDA(cudaGetLastError());
   team_kernel<K_DEC, 8><<<nd.team_grid, kTeamThreads, team_smem_bytes<K_DEC>(), st>>>(wa);
   RFD_CUDA(cudaGetLastError());
   noalloc_emit_kernel<<<1, 32, 0, st>>>(dstate, wa.error, right_ub);

@@ -1,0 +1,1274 @@
+// "Walk" sweeps: the pruned DFD, VE-FD and decision DPs of a pair, block by block along its
+// live band.
+//
+// At a level near its result a DP's live region is a thin band: on the uneven batch's pairs
+// and on the 200,000-point pair it crosses an anti-diagonal in 1.5 to 10 cells and one or two
+// blocks of 32 x 32 cells, whatever the curves' lengths.  The team strips (rfd_team.cuh) hand
+// a row on from one 32-row strip to the next through L2 in 32-column chunks, which costs such
+// a band about 11 us a strip.  Here one CTA walks the band instead:
+//   warp 0 (propagator)    goes through the 32-row block rows in order and, in each, through
+//                          the blocks that have a live input, left to right, one row at a time
+//                          (lane = column): the row below is a short list of live 32-column
+//                          chunks in shared memory, the column to the left one value per row;
+//   warps 1..7 (helpers)   compute the block's cell values into a tile: a cheap test (point
+//                          distance against the level plus a segment length) leaves the edges
+//                          that can be live, which are listed and evaluated densely.  Values
+//                          are kept in list order; per row, bit masks say which edges are
+//                          listed and which came out live, so nothing is stored for the rest.
+// While a block is swept the helpers fill the tile of the block most likely to be next (right
+// when an edge of the last column is live, up otherwise).  The grid's rows run along the longer
+// curve: a denser curve then moves the band up, which is the cheap direction of a row sweep.
+//
+// Exactness: a cell is skipped only when both its inputs are dead, an edge only when its value
+// is certainly dead (empty interval, weight above the pruning bound), the rules of the pruned
+// strips (rfd_device.cuh).  Live values are computed by the same functions from the same
+// operands and combined by exact min, max and comparisons, so results are bit-identical, and
+// the transposed grid gives the same values as for the strips (PairDesc::tr).
+//
+// Several CTAs share a long pair (a group): each walks a piece of the block rows.  Only the
+// first knows the row its piece starts from, so the others start from everything that could
+// be live there - every edge of that row with its free interval from its start, or its bare
+// weight - which can only be more live, or smaller, than the truth.  A thin band forgets its
+// start within a row or two: each piece is walked again from the end its predecessor came to,
+// but only until a block row's list equals the one the first walk recorded there; from there on
+// the first walk's is the true one.  For the min-max DPs "equals" is up to one constant: lists
+// with values max(c, v) against v stay so for good (min and max distribute), and the constants
+// of the pieces are combined at the end.  A piece that never meets its record hands its new
+// end on to another round, so the outcome does not rest on the band being forgetful, and a
+// piece that ends empty from everything that could be live ends the sweep (walk_sweep).  Once a
+// sweep has found the band, the next ones start their pieces only near where it ran.
+//
+// A sweep whose band is not thin (list overflow, block budget) gives up; the pair's phase then
+// runs on the strips as before.
+#pragma once
+
+#include "rfd_device.cuh"
+#include "rfd_filter.h"
+#include "rfd_team.cuh"
+
+namespace rfd {
+
+constexpr int kWalkHelpers = 7;
+constexpr int kWalkThreads = 32 * (kWalkHelpers + 1);
+constexpr int kWalkCap = 24;         // live chunks of a block row's output list
+constexpr double kDecDead = 4.0;     // dead decision value (live ones lie in [0, 1])
+constexpr double kDecLive = 2.0;     // below: live
+
+// Stage of a tile, in doubles: 33 points of each curve, then per row and per column the
+// segment's A, 0.5/A and skip threshold.
+constexpr int kWalkPts = 33 * 3;
+constexpr int kWalkStage = 2 * kWalkPts + 6 * 32;
+// Values of a tile, in double2: listed edges' intervals (decision), or doubles, two to an
+// entry (VE-FD weights; the DFD's point distances of all 1024 cells).  Rows that no longer fit
+// are left to a second tile of the block.
+constexpr int kWalkVals = 640;
+constexpr int kWalkFitRows = kWalkVals / 64;  // rows that fit whatever they list
+
+// A block row's output list as recorded by the first walk of a piece (n < 0: too long to record),
+// and the chunks lo .. hi of the list as last walked.
+constexpr int kWalkStretch = 10;
+constexpr int kWalkRec = 4;
+struct WalkRecord {
+  int n, lo, hi, pad;
+  int j[kWalkRec];
+  double v[kWalkRec][32];
+};
+struct WalkEnd {  // a piece's last list
+  int n, pad;
+  int j[kWalkCap];
+  double v[kWalkCap][32];
+};
+// What a member reports at the end of a round: constant and result of its piece, whether its end
+// changed in the round, which copy of the end is current (0: the first walk's, 1 or 2), whether
+// it is empty; part: the first walk did not start from everything, or lost something on the way.
+struct WalkStat {
+  double c, res;
+  int changed, which, empty, part, gave_up, pad;
+};
+// Points 32 J .. 32 J + 32 of a curve within rad of the centre (rad infinite: no bound).
+struct WalkBall {
+  double x[3], rad;
+};
+
+constexpr int kScan = -3;  // request word: the columns that can be live in the row below a piece
+
+struct WalkShared {
+  unsigned long long full[2];  // helpers -> propagator: tile ready
+  unsigned long long req[2];   // propagator -> helpers: tile requested
+  int req_i[2], req_j[2];      // block row (kStop: leave) and column
+  int req_r0[2], req_r1[2];    // rows of the block wanted
+  int cancel[2];               // the speculative tile is not needed
+  int cnt[2], fit[2];          // edges listed; entries that are (see walk_tile)
+  int rows[2];                 // the tile holds rows req_r0 .. rows - 1
+  PairDesc pd;                 // the running sweep's grid
+  int kind, flat, filter, mat;
+  double level, rad;           // pruning bound U or radius^2, and its root
+  unsigned long long cells, cells64;
+  uint4 mask[2][32];           // per row: listed right, listed top, live right, live top edges
+  int2 base[2][32];            // per row: first right edge's and first top edge's value
+  double bot[2][32];           // values rows enter / leave the block with
+  int up_j[2][kWalkCap];       // live chunks of the row below / of the row being made
+  double up_v[2][kWalkCap][32];
+  double stage[2][kWalkStage];
+  double2 vals[2][kWalkVals];
+  unsigned short list[2 * kWalkVals];
+  int nup, lost, scan_lo, scan_hi;  // scan of a piece's first row: chunks found, among which
+};
+constexpr size_t kWalkSmem = (sizeof(WalkShared) + 127) / 128 * 128;
+
+__device__ __forceinline__ void walk_helper_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * kWalkHelpers) : "memory");
+}
+
+// ------------------------------------------------------------------ helpers (warps 1..7)
+
+// Skip threshold of the edges of a segment with squared length A: an edge whose far end point
+// lies farther than this (squared) from the other curve's point is certainly dead.  The point
+// is then more than rad + 0.005 (rad + length) from every point of the segment, a relative
+// margin of 1e-6 of the squared distances involved, while the FP64 code that computes the
+// edge errs by about 1e-8 of them (a discriminant at 0) and never calls such an edge live.
+// No skipping for degenerate segments (their free interval is [0, 1] at any radius), near the
+// ends of the exponent range, or where distances are lost in the coordinates' rounding.
+__device__ __forceinline__ double walk_threshold(double rad, double A, double mag) {
+  if (!(A > 1e-200)) return (double)INFINITY;
+  const double s = rad + sqrt(A);
+  const double t = fmax(1.01 * s * s, 1e-14 * mag * mag);
+  return t < 1e200 ? t : (double)INFINITY;
+}
+
+// Tile of block (bi, bj), rows [r0, r1), all helpers; tid in [0, 32 H).  A row whose edges no
+// longer fit ends the tile: rows[slot] is the first such row, and the entries listed before
+// its place (fit[slot]) are the valid ones.
+template <int D>
+__device__ void walk_tile(const PairDesc& pd, WalkShared* sh, int slot, int bi, int bj, int r0,
+                          int r1, int tid) {
+  const int lane = tid & 31, hw = tid >> 5;
+  constexpr int NT = 32 * kWalkHelpers;
+  const int kind = sh->kind;
+  const bool dfd = kind == K_DFD;
+  double* P = sh->stage[slot];
+  double* Q = P + kWalkPts;
+  double* ra = Q + kWalkPts;  // row segments: A, 0.5/A, threshold
+  double* rinv = ra + 32;
+  double* rthr = rinv + 32;
+  double* ca = rthr + 32;     // column segments
+  double* cinv = ca + 32;
+  double* cthr = cinv + 32;
+  const int R = dfd ? pd.n1 : pd.n1 - 1, C = dfd ? pd.n2 : pd.n2 - 1;
+  const int i0 = bi << 5, j0 = bj << 5;
+  const int nr = min(r1, R - i0), nc = min(32, C - j0);
+  {
+    // points 32 bi .. 32 bi + 32 (clamped to the curve's end; clamped ones feed no cell)
+    const long long pe = (long long)pd.n1 * D, qe = (long long)pd.n2 * D;
+    for (int e = tid; e < 33 * D; e += NT) {
+      P[e] = __ldg(pd.P + min((long long)i0 * D + e, pe - 1));
+      Q[e] = __ldg(pd.Q + min((long long)j0 * D + e, qe - 1));
+    }
+  }
+  if (tid < 32) {
+    sh->mask[slot][tid] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) {
+      sh->cnt[slot] = 0;
+      sh->fit[slot] = INT_MAX;
+      sh->rows[slot] = r1;
+    }
+  }
+  if (!dfd && hw >= kWalkHelpers - 2) {
+    // segment constants as prep_kernel forms them (|p - q|^2 does not depend on the order)
+    const bool col = hw == kWalkHelpers - 1;
+    const double* X = col ? pd.Q : pd.P;
+    const double* x = X + (size_t)min((col ? j0 : i0) + lane, (col ? C : R) - 1) * D;
+    double t[D], mag = 0.0;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      const double b = __ldg(x + D + k);
+      t[k] = __dsub_rn(b, __ldg(x + k));
+      mag = fmax(mag, fabs(b));
+    }
+    const double A = sq_sum<D>(t);
+    double* a = col ? ca : ra;
+    a[lane] = A;
+    a[32 + lane] = __ddiv_rn(0.5, A);
+    a[64 + lane] = walk_threshold(sh->rad, A, mag);
+  }
+  walk_helper_sync();
+
+  if (dfd) {
+    // point distances are cheap: every cell
+    double* W = reinterpret_cast<double*>(sh->vals[slot]);
+    const double U = sh->level;
+    for (int r = r0 + hw; r < nr; r += kWalkHelpers) {
+      const double w = dist_sq<D>(P + r * D, Q + lane * D);
+      W[r * 32 + lane] = w;
+      const unsigned m = __ballot_sync(kFull, lane < nc && w <= U);
+      if (lane == 0) sh->mask[slot][r].w = m;
+    }
+    return;
+  }
+
+  // which edges can be live: lane = column
+  unsigned cells = 0, cells64 = 0;
+  const bool filt = kind == K_DEC && sh->filter;
+  const int cap = kind == K_DEC ? kWalkVals : 2 * kWalkVals;
+  {
+    double q[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) q[k] = Q[(lane + 1) * D + k];
+    const double ct = cthr[lane];
+    const unsigned lt = (1u << lane) - 1u;
+    // the warp's rows r0 + hw + 7 m together (independent tests), then one allocation for all
+    constexpr int M = (32 + kWalkHelpers - 1) / kWalkHelpers;
+    unsigned br[M], bt[M];
+    int n = 0;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int r = min(r0 + hw + m * kWalkHelpers, 31);
+      const bool in = lane < nc && r0 + hw + m * kWalkHelpers < nr;
+      const double s = dist_sq<D>(P + (r + 1) * D, q);
+      br[m] = __ballot_sync(kFull, in && (!(s > ct) || !(s < 1e200)));
+      bt[m] = __ballot_sync(kFull, in && (!(s > rthr[r]) || !(s < 1e200)));
+      n += __popc(br[m]) + __popc(bt[m]);
+      cells += __popc(br[m] | bt[m]);
+    }
+    if (n) {
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&sh->cnt[slot], n);
+      at = bcast(at);
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int r = r0 + hw + m * kWalkHelpers;
+        const int kr = __popc(br[m]), kt = __popc(bt[m]);
+        if (kr + kt == 0) continue;
+        if (at + kr + kt > cap) {
+          if (lane == 0) {
+            atomicMin(&sh->rows[slot], r);
+            atomicMin(&sh->fit[slot], at);
+          }
+        } else {
+          if (br[m] >> lane & 1u) sh->list[at + __popc(br[m] & lt)] = (unsigned short)(r << 5 | lane);
+          if (bt[m] >> lane & 1u)
+            sh->list[at + kr + __popc(bt[m] & lt)] = (unsigned short)(1024 | r << 5 | lane);
+          if (lane == 0) {
+            sh->mask[slot][r] = make_uint4(br[m], bt[m], 0u, 0u);
+            sh->base[slot][r] = make_int2(at, at + kr);
+          }
+        }
+        at += kr + kt;
+      }
+    }
+  }
+  if (lane == 0 && cells) atomicAdd(&sh->cells, (unsigned long long)cells);
+  walk_helper_sync();
+
+  const int cnt = min(sh->cnt[slot], sh->fit[slot]);
+  const double level = sh->level;
+  const bool mat = sh->mat != 0;
+  if (*(volatile int*)&sh->cancel[slot]) return;
+  for (int k = tid; k < cnt; k += NT) {
+    const int e = sh->list[k], cell = e & 1023, r = cell >> 5, c = cell & 31;
+    const bool top = e >= 1024;
+    // right edge: p_{i+1} against q_j q_{j+1}; top edge: q_{j+1} against p_i p_{i+1}
+    const double* x = top ? Q + (c + 1) * D : P + (r + 1) * D;
+    const double* a = top ? P + r * D : Q + c * D;
+    double di[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) di[d] = __dsub_rn(a[D + d], a[d]);
+    const double A = top ? ra[r] : ca[c];
+    bool live;
+    if (kind == K_DEC) {
+      double lo, hi;
+      // the FP32 filter's certain answers need no FP64 (rfd_filter.h)
+      const int cls = filt ? interval_class32<D>(x, a, di, A, level) : 0;
+      if (cls == 0) {
+        free_interval<D>(x, a, di, A, top ? rinv[r] : cinv[c], level, lo, hi, mat);
+        if (filt) ++cells64;
+      } else {
+        lo = cls == 1 ? -1.0 : 0.0;
+        hi = cls == 1 ? -2.0 : 1.0;
+      }
+      sh->vals[slot][k] = make_double2(lo, hi);
+      live = !(lo < 0.0);
+    } else {
+      const double w = pt_seg_sq<D>(x, a, di, A);
+      reinterpret_cast<double*>(sh->vals[slot])[k] = w;
+      live = w <= level;
+    }
+    if (live) atomicOr(top ? &sh->mask[slot][r].w : &sh->mask[slot][r].z, 1u << c);
+  }
+  // (edges, halved: at most the cells listed)
+  if (cells64) atomicAdd(&sh->cells64, (unsigned long long)cells64);
+}
+
+// Bounds of a curve's chunks (points 32 J - 1 .. 32 J + 32), one warp a chunk; a chunk with a
+// degenerate segment, whose free interval is [0, 1] at any radius, is unbounded.
+template <int D>
+__device__ void walk_ball(const double* X, int n, int j, WalkBall* out) {
+  const int lane = threadIdx.x & 31;
+  double lo[D], hi[D];
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    lo[k] = (double)INFINITY;
+    hi[k] = -(double)INFINITY;
+  }
+  bool odd = false;
+  for (int q = (j << 5) - 1 + lane; q <= (j << 5) + 32; q += 32) {
+    if (q < 0 || q >= n) continue;
+    double A = 0.0;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      const double v = X[(size_t)q * D + k];
+      lo[k] = fmin(lo[k], v);
+      hi[k] = fmax(hi[k], v);
+      odd |= !(fabs(v) < 1e140);
+      if (q + 1 < n) {
+        const double d = X[(size_t)(q + 1) * D + k] - v;
+        A += d * d;
+      }
+    }
+    if (q + 1 < n) odd |= !(A > 1e-200);
+  }
+  double rad = 0.0, x[D];
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[k] = fmin(lo[k], __shfl_xor_sync(kFull, lo[k], o));
+      hi[k] = fmax(hi[k], __shfl_xor_sync(kFull, hi[k], o));
+    }
+    x[k] = 0.5 * (lo[k] + hi[k]);
+    rad += 0.25 * (hi[k] - lo[k]) * (hi[k] - lo[k]);
+  }
+  odd = __any_sync(kFull, odd);
+  if (lane == 0) {
+    WalkBall b;
+    b.x[2] = 0.0;
+#pragma unroll
+    for (int k = 0; k < D; ++k) b.x[k] = x[k];
+    b.rad = odd ? (double)INFINITY : 1.000001 * sqrt(rad);
+    *out = b;
+  }
+}
+
+// The row below block row bi, as far as it can be live (see the head comment): chunks into list
+// `to`, in no order (the propagator sorts them); sh->nup of them, sh->lost if some did not fit.
+template <int D>
+__device__ void walk_scan(const PairDesc& pd, WalkShared* sh, int to, int bi, int tid) {
+  const int lane = tid & 31, hw = tid >> 5;
+  const int kind = sh->kind;
+  const bool dfd = kind == K_DFD;
+  const int C = dfd ? pd.n2 : pd.n2 - 1, nbc = (C + 31) >> 5;
+  const double level = sh->level;
+  if (tid == 0) sh->nup = sh->lost = 0;
+  walk_helper_sync();
+  // segment kinds: point 32 bi against the columns' segments; DFD: point 32 bi - 1
+  const double* xp = pd.P + (size_t)((bi << 5) - (dfd ? 1 : 0)) * D;
+  double x[D];
+  double mag = 0.0;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    x[k] = __ldg(xp + k);
+    mag = fmax(mag, fabs(x[k]));
+  }
+  const double dead = kind == K_DEC ? kDecDead : kFltMax;
+  const int j1 = min(nbc, sh->scan_hi + 1);
+  for (int jb = max(0, sh->scan_lo) + 32 * hw; jb < j1; jb += 32 * kWalkHelpers) {
+   // 32 chunks' bounds at once, then the chunks in reach one by one
+   bool reach = false;
+   if (jb + lane < j1) {
+    const WalkBall* b = pd.balls + jb + lane;
+    double t[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) t[k] = x[k] - __ldg(&b->x[k]);
+    const double far = 1.00001 * (sh->rad + __ldg(&b->rad)) + 1e-7 * mag;
+    reach = !(sq_sum<D>(t) > far * far);
+   }
+   unsigned todo = __ballot_sync(kFull, reach);
+   while (todo) {
+    const int j = jb + __ffs(todo) - 1, c = (j << 5) + lane;
+    todo &= todo - 1;
+    double v = dead;
+    if (c < C) {
+      if (dfd) {
+        auto weight = [&](int q) {
+          double b[D];
+#pragma unroll
+          for (int e = 0; e < D; ++e) b[e] = __ldg(pd.Q + (size_t)q * D + e);
+          return dist_sq<D>(x, b);
+        };
+        const double w = weight(c), l = weight(max(c - 1, 0));
+        v = l < w ? l : w;
+        v = v <= level ? v : dead;
+      } else {
+        double a[D], di[D];
+#pragma unroll
+        for (int e = 0; e < D; ++e) {
+          a[e] = __ldg(pd.Q + (size_t)c * D + e);
+          di[e] = __dsub_rn(__ldg(pd.Q + (size_t)(c + 1) * D + e), a[e]);
+        }
+        const double A = sq_sum<D>(di);
+        if (kind == K_DEC) {
+          double lo, hi;
+          free_interval<D>(x, a, di, A, __ddiv_rn(0.5, A), level, lo, hi, sh->mat != 0);
+          v = lo < 0.0 ? dead : lo;
+        } else {
+          const double w = pt_seg_sq<D>(x, a, di, A);
+          v = w <= level ? w : dead;
+        }
+      }
+    }
+    if (sh->flat && v < dead) v = 0.0;
+    if (!__any_sync(kFull, v < (kind == K_DEC ? kDecLive : kFltMax))) continue;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&sh->nup, 1);
+    at = bcast(at);
+    if (at < kWalkCap) {
+      sh->up_v[to][at][lane] = v;
+      if (lane == 0) sh->up_j[to][at] = j;
+    } else if (lane == 0) {
+      sh->lost = 1;
+    }
+   }
+  }
+}
+
+// Helper warps: tiles as requested, until kStop.
+__device__ void walk_helpers(const WaveArgs& wa, WalkShared* sh) {
+  const int tid = threadIdx.x - 32, lane = tid & 31;
+  unsigned seq = 0;
+  for (;;) {
+    const int slot = seq & 1;
+    if (!mbar_wait(&sh->req[slot], (seq >> 1) & 1, wa, clock64())) break;
+    const int bi = *(volatile int*)&sh->req_i[slot], bj = *(volatile int*)&sh->req_j[slot];
+    if (bi == kStop) break;
+    const int r0 = *(volatile int*)&sh->req_r0[slot], r1 = *(volatile int*)&sh->req_r1[slot];
+    const PairDesc pd = sh->pd;
+    if (bi == kScan) {
+      if (pd.d == 2) walk_scan<2>(pd, sh, r0, bj, tid);
+      else walk_scan<3>(pd, sh, r0, bj, tid);
+    } else if (pd.d == 2) walk_tile<2>(pd, sh, slot, bi, bj, r0, r1, tid);
+    else walk_tile<3>(pd, sh, slot, bi, bj, r0, r1, tid);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh->full[slot]);
+    ++seq;
+  }
+}
+
+// ------------------------------------------------------------------ propagator (warp 0)
+
+template <int KIND>
+__device__ __forceinline__ double walk_dead() {
+  return KIND == K_DEC ? kDecDead : kFltMax;
+}
+// Live values are below the dead one by construction (masked edges only); for the decision the
+// high word decides.
+template <int KIND>
+__device__ __forceinline__ bool walk_live(double v) {
+  return KIND == K_DEC ? __double2hiint(v) < __double2hiint(kDecLive) : v < kFltMax;
+}
+// a < b for values >= 0 (or -0, which sorts first) as integers: shorter than an FP64 compare.
+__device__ __forceinline__ bool walk_less(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+
+__device__ __forceinline__ double walk_min(double a, double b) { return walk_less(a, b) ? a : b; }
+__device__ __forceinline__ double walk_max(double a, double b) { return walk_less(a, b) ? b : a; }
+
+// One row's tile words for this lane's column, in the two dependent steps they load in: the
+// row's masks and places, then the values and (decision) what the left neighbour would pass on.
+struct WalkHead {
+  uint4 m;
+  int2 base;
+};
+struct WalkRow {
+  unsigned mr, mt;  // live right / top edges of the row
+  double2 r, t;     // their values (VE-FD: weights in .x; DFD: t.x)
+};
+template <int KIND>
+__device__ __forceinline__ WalkHead walk_row_head(const WalkShared* sh, int slot, int r) {
+  WalkHead h;
+  h.m = sh->mask[slot][r];
+  if (KIND != K_DFD) h.base = sh->base[slot][r];
+  return h;
+}
+template <int KIND>
+__device__ __forceinline__ WalkRow walk_row_load(const WalkShared* sh, int slot, int r,
+                                                 const WalkHead& h, bool flat) {
+  const int lane = threadIdx.x & 31;
+  WalkRow w;
+  w.mr = h.m.z;
+  w.mt = h.m.w;
+  if (KIND == K_DFD) {
+    const double t = reinterpret_cast<const double*>(sh->vals[slot])[r * 32 + lane];
+    w.t.x = flat ? 0.0 : t;
+  } else {
+    // (a lane without a listed edge reads another's value and does not use it; the places of a
+    // row that lists nothing are stale, hence the bound)
+    const unsigned lt = (1u << lane) - 1u;
+    constexpr unsigned cap = (KIND == K_DEC ? kWalkVals : 2 * kWalkVals) - 1;
+    const unsigned kr = min((unsigned)h.base.x + __popc(h.m.x & lt), cap);
+    const unsigned kt = min((unsigned)h.base.y + __popc(h.m.y & lt), cap);
+    if (KIND == K_DEC) {
+      w.r = sh->vals[slot][kr];
+      w.t = sh->vals[slot][kt];
+    } else {
+      const double a = reinterpret_cast<const double*>(sh->vals[slot])[kr];
+      const double b = reinterpret_cast<const double*>(sh->vals[slot])[kt];
+      w.r.x = flat ? 0.0 : a;
+      w.t.x = flat ? 0.0 : b;
+    }
+  }
+  return w;
+}
+// Decision: the value the column to the left passes on when it is live from below (lane 0: the
+// value the row enters with), and the columns whose top edge ends before it.
+struct WalkPrev {
+  double v;
+  unsigned late;
+};
+__device__ __forceinline__ WalkPrev walk_row_prev(const WalkRow& w, double x0) {
+  WalkPrev p;
+  p.v = __shfl_up_sync(kFull, w.t.x, 1);
+  p.v = (threadIdx.x & 31) == 0 ? x0 : p.v;
+  p.late = __ballot_sync(kFull, __double_as_longlong(w.t.y) < __double_as_longlong(p.v));
+  return p;
+}
+
+// One row of a block (lane = column).  F: value handed up by the row below, replaced by this
+// row's; V: its live columns.  in: whether the row enters the block live, with value x0.  y:
+// value this lane's column hands to the right; Y: the columns that hand on a live one.
+//
+// Decision.  The value runs right through top edges: column j hands on t.lo when it is live
+// from below, else max(t.lo, x) if the incoming x is at most t.hi.  Whether a value arrives is
+// a carry chain of bits (generate: live from below and the edge free; propagate: edge free),
+// one addition for the row - exact unless a value that passed a column without support from
+// below meets an edge that ends before it.  The value such a pass brings is the previous
+// column's t.lo when the pass is one column long, so one comparison settles those; longer
+// passes, and comparisons that fail, go column by column (the band is a few cells wide: rare).
+template <int KIND>
+__device__ __forceinline__ void walk_row(const WalkRow& w, const WalkPrev& pv, bool in, double x0,
+                                         double& F, unsigned& V, double& y, unsigned& Y) {
+  const int lane = threadIdx.x & 31;
+  const unsigned bit = 1u << lane;
+  const double dead = walk_dead<KIND>();
+  const bool br = (w.mr & bit) != 0u, bt = (w.mt & bit) != 0u;
+  const double first = in ? x0 : dead;  // what enters column 0
+  if (KIND == K_DEC) {
+    const unsigned gen = V & w.mt;
+    unsigned X = (w.mt + gen + (unsigned)in) ^ w.mt ^ gen;  // live values arriving at a column
+    const unsigned pass = X & ~V & w.mt;
+    const bool up = (V & bit) != 0u;
+    const bool reset = up | !walk_less(w.t.x, pv.v);
+    y = reset ? w.t.x : pv.v;
+    Y = w.mt & (V | X);
+    if (pass & (pv.late | (pass << 1))) {
+      double x;
+      y = bt & up ? w.t.x : dead;
+      for (;;) {
+        x = __shfl_up_sync(kFull, y, 1);
+        x = lane == 0 ? first : x;
+        const bool ends = !bt | (!up & walk_less(w.t.y, x));
+        const bool own = up | !walk_less(w.t.x, x);
+        double yn = own ? w.t.x : x;
+        yn = ends ? dead : yn;
+        const bool moved = walk_less(yn, y) | walk_less(y, yn);
+        y = yn;
+        if (!__any_sync(kFull, moved)) break;
+      }
+      X = __ballot_sync(kFull, walk_live<KIND>(x));
+      Y = __ballot_sync(kFull, walk_live<KIND>(y));
+    }
+    const bool xl = (X & bit) != 0u;
+    const bool ok = br & (xl | !walk_less(w.r.y, F));
+    const bool own = xl | !walk_less(w.r.x, F);
+    const double f = own ? w.r.x : F;
+    F = ok ? f : dead;
+    V = __ballot_sync(kFull, ok);
+  } else {
+    // y_j = max(w_j, min(F_j, y_{j-1})): from the values entering from below, repeated while a
+    // changed column has a live right neighbour (as often as the longest run of cells reached
+    // from the left)
+    double x = lane == 0 ? first : dead;
+    y = walk_max(w.t.x, walk_min(F, x));
+    y = bt ? y : dead;
+    for (;;) {
+      x = __shfl_up_sync(kFull, y, 1);
+      x = lane == 0 ? first : x;
+      double yn = walk_max(w.t.x, walk_min(F, x));
+      yn = bt ? yn : dead;
+      const unsigned moved = __ballot_sync(kFull, walk_less(yn, y));
+      y = yn;
+      if ((moved << 1) & w.mt) continue;
+      if (moved) {
+        x = __shfl_up_sync(kFull, y, 1);
+        x = lane == 0 ? first : x;
+      }
+      break;
+    }
+    if (KIND == K_DFD) {
+      F = walk_min(y, x);
+    } else {
+      const double f = walk_max(w.r.x, walk_min(F, x));
+      F = br ? f : dead;
+    }
+    V = __ballot_sync(kFull, walk_live<KIND>(F));
+    Y = __ballot_sync(kFull, walk_live<KIND>(y));
+  }
+}
+
+// Walk of one CTA: requests outstanding, and the list of the row below.
+struct Walk {
+  unsigned seq_p, seq_c;  // tiles requested, taken
+  int pi, pj, pr;         // the outstanding request (pi < 0: none)
+  int cur, n;             // list of the row below: buffer and live chunks
+  long long blocks;       // blocks swept
+  int rec_from, rec_end;  // block rows whose records this sweep can be met at
+  // where an earlier sweep's band ran: this member's piece, cut so that pieces take equal
+  // stretches of the band (cut0 < 0: equal block rows), and the chunks it entered it in (lo > hi:
+  // not known)
+  int cut0, cut1, near_lo, near_hi;
+  int rounds;             // rounds of this phase's sweeps beyond each one's first two
+};
+
+enum WalkStatus : int { WALK_OK = 0, WALK_ERROR, WALK_GIVE_UP, WALK_MET, WALK_UNSETTLED };
+// How a piece is walked: alone (the whole grid); the first time from what could be live, or
+// from the true start, recording every block row's list; again, until it meets a record.
+enum WalkMode : int { WALK_ALONE = 0, WALK_RECORD = 1, WALK_AGAIN = 2 };
+
+__device__ __forceinline__ void walk_request(WalkShared* sh, Walk& w, int i, int j, int r0 = 0,
+                                             int r1 = 32) {
+  if ((threadIdx.x & 31) == 0) {
+    const int slot = w.seq_p & 1;
+    *(volatile int*)&sh->req_i[slot] = i;
+    *(volatile int*)&sh->req_j[slot] = j;
+    *(volatile int*)&sh->req_r0[slot] = r0;
+    *(volatile int*)&sh->req_r1[slot] = r1;
+    *(volatile int*)&sh->cancel[slot] = 0;
+    mbar_arrive(&sh->req[slot]);
+  }
+  __syncwarp();
+  ++w.seq_p;
+  w.pi = i;
+  w.pj = j;
+  w.pr = r0;
+}
+// The propagator's wait for a tile (bounded).  It polls: the helpers' waits suspend
+// (mbarrier.try_wait), but this one is on the sweep's chain.
+__device__ __forceinline__ bool walk_wait(unsigned long long* b, unsigned parity, const WaveArgs& wa) {
+  const long long t0 = clock64();
+  for (int it = 0;; ++it) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_addr(b)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    int bad = 0;
+    if ((threadIdx.x & 31) == 0)
+      bad = clock64() - t0 > wa.spin_cycles || ((it & 255) == 255 && ld_volatile(wa.error));
+    if (__shfl_sync(kFull, bad, 0)) {
+      if ((threadIdx.x & 31) == 0) atomicExch(wa.error, 1);
+      return false;
+    }
+  }
+}
+// Waits for the outstanding tile; its slot, or -1 on an error.
+__device__ __forceinline__ int walk_take(const WaveArgs& wa, WalkShared* sh, Walk& w) {
+  const int slot = w.seq_c & 1;
+  if (!walk_wait(&sh->full[slot], (w.seq_c >> 1) & 1, wa)) return -1;
+  ++w.seq_c;
+  w.pi = -1;
+  return slot;
+}
+__device__ __forceinline__ bool walk_drop(const WaveArgs& wa, WalkShared* sh, Walk& w) {
+  if (w.pi < 0) return true;
+  if ((threadIdx.x & 31) == 0) *(volatile int*)&sh->cancel[w.seq_c & 1] = 1;
+  __syncwarp();
+  return walk_take(wa, sh, w) >= 0;
+}
+// The tile of block (i, j) from row r0 on: taken if it is the outstanding request.
+__device__ __forceinline__ int walk_get(const WaveArgs& wa, WalkShared* sh, Walk& w, int i, int j,
+                                        int r0, int r1 = 32) {
+  if (w.pi != i || w.pj != j || w.pr != r0) {
+    if (!walk_drop(wa, sh, w)) return -1;
+    walk_request(sh, w, i, j, r0, r1);
+  }
+  return walk_take(wa, sh, w);
+}
+
+// Sweeps block rows [i0, i1) from the row below (w.cur, w.n); start: the value the grid's
+// first row enters column 0 with (dead: none).  On return the list holds the last row's
+// output; res is set when the grid's last cell was reached.
+// Recording, chunks that do not fit the list are dropped if `loose` (lost is set).  Walking
+// again, WALK_MET says that a block row's list equals its record up to the constant c.
+template <int KIND>
+__device__ int walk_rows(const WaveArgs& wa, WalkShared* sh, Walk& w, int i0, int i1, double start,
+                         double& res, WalkMode mode, WalkRecord* recs, bool loose, bool& lost,
+                         double& c) {
+  const int lane = threadIdx.x & 31;
+  const double dead = walk_dead<KIND>();
+  const int R = KIND == K_DFD ? sh->pd.n1 : sh->pd.n1 - 1;
+  const int C = KIND == K_DFD ? sh->pd.n2 : sh->pd.n2 - 1;
+  const int nbr = (R + 31) >> 5, nbc = (C + 31) >> 5;
+  const bool flat = KIND != K_DEC && sh->flat;
+  int j_min = INT_MAX, j_max = 0;
+  int status = WALK_OK;
+  for (int i = i0; i < i1 && status == WALK_OK; ++i) {
+    const int in = w.cur, ob = w.cur ^ 1;
+    const int nr = min(32, R - (i << 5));
+    // the record to compare with, loaded while the row is walked
+    int rec_n = -1, rec_j = 0;
+    double rec_v[kWalkRec];
+    if (mode == WALK_AGAIN) {
+      const WalkRecord* q = recs + i;
+      rec_n = __ldcg(&q->n);
+      if (lane < kWalkRec) rec_j = __ldcg(&q->j[lane]);
+#pragma unroll
+      for (int e = 0; e < kWalkRec; ++e) rec_v[e] = __ldcg(&q->v[e][lane]);
+    }
+    int k = 0, on = 0, j = -1;
+    unsigned bmask = 0u;  // rows that enter the next block live, values in sh->bot[bb]
+    int bb = 0;
+    if (i == 0 && walk_live<KIND>(start)) {
+      bmask = 1u;
+      j = 0;
+      if (lane == 0) sh->bot[0][0] = start;
+      __syncwarp();
+    }
+    while (status == WALK_OK) {
+      if (j < 0) {
+        if (k >= w.n) break;
+        j = sh->up_j[in][k];
+      }
+      const bool have = k < w.n && sh->up_j[in][k] == j;
+      double F = have ? sh->up_v[in][k][lane] : dead;
+      unsigned V = __ballot_sync(kFull, walk_live<KIND>(F));
+      k += have;
+      int slot = walk_get(wa, sh, w, i, j, 0);
+      if (slot < 0) { status = WALK_ERROR; break; }
+      // effort against progress: a thin band lists a few hundred edges a block and goes from block
+      // to block right or up
+      w.blocks += 1 + (sh->cnt[slot] >> 8);
+      j_min = min(j_min, j);
+      j_max = max(j_max, j);
+      if (w.blocks > 64 + 4LL * ((i - i0) + (j_max - j_min)) || (on == kWalkCap && !loose)) {
+        status = WALK_GIVE_UP;
+        break;
+      }
+      int rows = *(volatile int*)&sh->rows[slot];
+      {
+        // the next block: right when this one's last column has a live edge, else the next
+        // chunk of the row, else up
+        const uint4 m = sh->mask[slot][lane];
+        const bool right = __any_sync(kFull, m.w >> 31);
+        const bool more = k < w.n;
+        int ni = -1, nj = 0;
+        if (rows < nr) {
+          // (this block's other rows come first)
+        } else if (j + 1 < nbc && (right || (more && sh->up_j[in][k] == j + 1))) {
+          ni = i;
+          nj = j + 1;
+        } else if (more) {
+          ni = i;
+          nj = sh->up_j[in][k];
+        } else if (i + 1 < i1) {
+          ni = i + 1;
+          nj = on ? sh->up_j[ob][0] : j;
+        }
+        if (ni >= 0) walk_request(sh, w, ni, nj);
+      }
+      const bool last = i == nbr - 1 && j == nbc - 1;
+      unsigned omask = 0u;
+      const double* bin = sh->bot[bb];
+      double* bout = sh->bot[bb ^ 1];
+      int r = 0;
+      while (true) {
+        if (V == 0u) {
+          // nothing from below: on to the next row that enters live, if any
+          const unsigned left = r < 32 ? bmask & (0xffffffffu << r) : 0u;
+          if (!left) { r = nr; break; }
+          r = __ffs(left) - 1;
+        }
+        if (r >= nr) break;
+        if (r >= rows) {
+          slot = walk_get(wa, sh, w, i, j, r);
+          if (slot >= 0 && *(volatile int*)&sh->rows[slot] <= r)
+            slot = walk_get(wa, sh, w, i, j, r, min(32, r + kWalkFitRows));
+          if (slot < 0) { status = WALK_ERROR; break; }
+          rows = *(volatile int*)&sh->rows[slot];
+        }
+        // rows r .. stop - 1, their loads two and one rows ahead
+        const int stop = min(rows, nr);
+        auto enter = [&](int q) { return bin[min(q, 31)]; };
+        WalkRow cur = walk_row_load<KIND>(sh, slot, r, walk_row_head<KIND>(sh, slot, r), flat);
+        WalkHead head = walk_row_head<KIND>(sh, slot, min(r + 1, 31));
+        double x0 = enter(r);
+        WalkPrev pv;
+        if (KIND == K_DEC) pv = walk_row_prev(cur, x0);
+        double y;
+        unsigned Y;
+        WalkRow at;
+        do {
+          const WalkRow nxt = walk_row_load<KIND>(sh, slot, min(r + 1, 31), head, flat);
+          head = walk_row_head<KIND>(sh, slot, min(r + 2, 31));
+          const double x1 = enter(r + 1);
+          walk_row<KIND>(cur, pv, (bmask >> r) & 1u, x0, F, V, y, Y);
+          if ((lane == 31) & (int)(Y >> 31)) bout[r] = y;
+          omask |= (Y >> 31) << r;
+          if (KIND == K_DEC) pv = walk_row_prev(nxt, x1);
+          at = cur;
+          cur = nxt;
+          x0 = x1;
+          ++r;
+        } while ((r < stop) & (V != 0u));
+        if (last && r == nr) {
+          // the last cell: VE-FD the lesser of its edges, DFD its value; the decision its right
+          // edge's upper end (top edge on a transposed grid) if that edge is reached
+          const int cl = (C - 1) & 31;
+          double v;
+          if (KIND == K_DEC) {
+            const bool tr = sh->pd.tr != 0;
+            v = ((tr ? Y : V) >> cl) & 1u ? (tr ? at.t.y : at.r.y) : -2.0;
+          } else {
+            v = KIND == K_VEFD ? dmin(y, F) : y;
+          }
+          res = __shfl_sync(kFull, v, cl);
+        }
+      }
+      if (status != WALK_OK) break;
+      if (V && i + 1 < nbr) {
+        if (on < kWalkCap) {
+          sh->up_v[ob][on][lane] = F;
+          if (lane == 0) sh->up_j[ob][on] = j;
+          ++on;
+        } else {
+          lost = true;
+          w.rec_from = i + 1;  // (earlier records lead to more than what is walked on)
+        }
+      }
+      __syncwarp();
+      bmask = omask;
+      bb ^= 1;
+      j = omask && j + 1 < nbc ? j + 1 : -1;
+    }
+    w.cur = ob;
+    w.n = on;
+    if (status != WALK_OK) break;
+    if (mode != WALK_ALONE && on && lane == 0) {
+      __stcg(&recs[i].lo, sh->up_j[ob][0]);
+      __stcg(&recs[i].hi, sh->up_j[ob][on - 1]);
+    }
+    if (mode == WALK_RECORD) {
+      w.rec_end = i;
+      WalkRecord* q = recs + i;
+      const int n = on <= kWalkRec ? on : -1;
+      if (lane == 0) __stcg(&q->n, n);
+      if (lane < n) __stcg(&q->j[lane], sh->up_j[ob][lane]);
+      for (int e = 0; e < n; ++e) __stcg(&q->v[e][lane], sh->up_v[ob][e][lane]);
+    } else if (mode == WALK_AGAIN && i + 1 < nbr && i >= w.rec_from && i <= w.rec_end &&
+               rec_n == on) {
+      bool same = lane >= on || sh->up_j[ob][lane] == rec_j;
+      double m = 0.0;
+#pragma unroll
+      for (int e = 0; e < kWalkRec; ++e) {
+        if (e >= on) break;
+        const double v = sh->up_v[ob][e][lane];
+        if (KIND == K_DEC) same &= __double_as_longlong(v) == __double_as_longlong(rec_v[e]);
+        else if (v != rec_v[e]) m = fmax(m, v);
+      }
+      if (KIND != K_DEC) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(kFull, m, o));
+#pragma unroll
+        for (int e = 0; e < kWalkRec; ++e) {
+          if (e >= on) break;
+          const double v = sh->up_v[ob][e][lane];
+          same &= v == fmax(m, rec_v[e]) && walk_live<KIND>(v) == walk_live<KIND>(rec_v[e]);
+        }
+      }
+      if (__all_sync(kFull, same)) {
+        c = m;
+        status = WALK_MET;
+      }
+    }
+    if (on == 0) break;
+  }
+  if (!walk_drop(wa, sh, w)) status = WALK_ERROR;
+  __syncwarp();
+  return status;
+}
+
+// The group of CTAs that walks a pair: `size` of them, this one is `rank`; members' reports and
+// ends are at `first` + rank of the arrays.
+struct WalkGroup {
+  int size, rank, first;
+  unsigned passed;        // barriers passed
+  unsigned* arrive;       // the group's arrival count
+  WalkStat* stat[2];      // by round
+  WalkEnd* end[3];
+};
+
+// Barrier of the group's propagators (bounded).  All CTAs of the launch are co-resident
+// (cooperative launch).  false on an error.
+__device__ __forceinline__ bool walk_barrier(const WaveArgs& wa, WalkGroup& g) {
+  ++g.passed;
+  if (g.size == 1) return true;
+  __syncwarp();
+  int bad = 0;
+  if ((threadIdx.x & 31) == 0) {
+    __threadfence();
+    atomicAdd(g.arrive, 1u);
+    const unsigned want = g.passed * (unsigned)g.size;
+    const long long t0 = clock64();
+    for (int it = 0;; ++it) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g.arrive) : "memory");
+      if (v >= want) break;
+      if ((it & 15) == 15 && (ld_volatile(wa.error) || clock64() - t0 > wa.spin_cycles)) {
+        atomicExch(wa.error, 1);
+        bad = 1;
+        break;
+      }
+    }
+    __threadfence();
+  }
+  return !bcast(bad);
+}
+
+__device__ __forceinline__ void walk_save_end(const WalkShared* sh, const Walk& w, WalkEnd* e) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) __stcg(&e->n, w.n);
+  if (lane < w.n) __stcg(&e->j[lane], sh->up_j[w.cur][lane]);
+  for (int k = 0; k < w.n; ++k) __stcg(&e->v[k][lane], sh->up_v[w.cur][k][lane]);
+}
+__device__ __forceinline__ void walk_load_end(WalkShared* sh, Walk& w, const WalkEnd* e) {
+  const int lane = threadIdx.x & 31;
+  w.cur = 0;
+  w.n = __ldcg(&e->n);
+  if (lane < w.n) sh->up_j[0][lane] = __ldcg(&e->j[lane]);
+  for (int k = 0; k < w.n; ++k) sh->up_v[0][k][lane] = __ldcg(&e->v[k][lane]);
+  __syncwarp();
+}
+
+// The list of everything that could be live in the row below block row i, sorted by column (near
+// the band of an earlier sweep, if there was one: not everything, then).
+__device__ bool walk_start_row(const WaveArgs& wa, WalkShared* sh, Walk& w, int i, bool& lost) {
+  const int lane = threadIdx.x & 31;
+  const bool near = w.near_lo <= w.near_hi;
+  if (lane == 0) {
+    sh->scan_lo = near ? w.near_lo - 2 : 0;
+    sh->scan_hi = near ? w.near_hi + 2 : INT_MAX - 1;
+  }
+  __syncwarp();
+  walk_request(sh, w, kScan, i, 1);
+  if (walk_take(wa, sh, w) < 0) return false;
+  const int n = min(*(volatile int*)&sh->nup, kWalkCap);
+  lost = near || *(volatile int*)&sh->lost != 0;
+  const int mine = lane < n ? sh->up_j[1][lane] : INT_MAX;
+  int rank = 0;
+  for (int k = 0; k < n; ++k) rank += __shfl_sync(kFull, mine, k) < mine;
+  if (lane < n) sh->up_j[0][rank] = mine;
+  for (int k = 0; k < n; ++k) sh->up_v[0][__shfl_sync(kFull, rank, k)][lane] = sh->up_v[1][k][lane];
+  w.cur = 0;
+  w.n = n;
+  __syncwarp();
+  return true;
+}
+
+// The piece of member m by where the band of an earlier sweep ran, from the records: block row i
+// ends about i + (its list's last chunk) blocks along it.  Pieces take equal stretches: piece q
+// starts with the first row that ends past q / pieces of the way (a bisection; the same for both
+// its neighbours, since no record changes meanwhile).
+__device__ void walk_cut(Walk& w, const WalkRecord* recs, int nbr, int nbc, int pieces, int m) {
+  const int lane = threadIdx.x & 31;
+  const int q = m + (lane & 1);  // lane 0: this piece's start, lane 1: its end
+  int lo = 0, hi = nbr;
+  const long long want = (long long)(nbr + nbc) * q / pieces;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if ((long long)mid + __ldcg(&recs[mid].hi) >= want) hi = mid;
+    else lo = mid + 1;
+  }
+  // (the band runs up and right, so these are in order; at least one row per piece)
+  lo = min(max(lo, q), nbr - pieces + q);
+  const int c0 = __shfl_sync(kFull, lo, 0), c1 = __shfl_sync(kFull, lo, 1);
+  w.cut0 = m == 0 ? 0 : c0;
+  w.cut1 = m + 1 >= pieces ? nbr : c1;
+  w.near_lo = 0;
+  w.near_hi = -1;
+  if (w.cut0 > 0) {
+    w.near_lo = __ldcg(&recs[w.cut0 - 1].lo);
+    w.near_hi = __ldcg(&recs[w.cut0 - 1].hi);
+  }
+}
+
+// The number of pieces of a grid: of at least kWalkStretch blocks of a thin band (shorter ones
+// end before the band has forgotten their start).
+__device__ __forceinline__ int walk_pieces(const PairDesc& pd, int size, int nbr, int nbc) {
+  return pd.recs ? max(1, min(min(size, nbr / 2), (nbr + nbc) / kWalkStretch)) : 1;
+}
+
+// Options of a sweep.  flat: only whether a path survives the level (every live value 0): its
+// lists meet their records as soon as the live columns do.  rounds: after so many it stops as
+// WALK_UNSETTLED.
+struct WalkSweep {
+  bool flat;
+  int rounds;
+  int limit;  // of Walk::rounds: past it the phase is given up
+  // out: the largest of the least values the pieces end with.  No path has less if the pieces
+  // started from everything that could be live (sure).
+  double least;
+  bool sure;
+  bool band;  // the sweep found a band: the records say where it ran
+};
+
+// A whole sweep of the grid in sh->pd at a level, by the group.  Returns a WalkStatus; res: the
+// DP's result (VE-FD and DFD: kFltMax when the level cuts every path; decision: -2 when
+// unreachable).  Every member gets the same answer; a barrier must follow before the next sweep
+// (reports, ends and records are free again once all have read them).
+template <int KIND>
+__device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup& g, double level,
+                          double rad, double seed, WalkSweep& o, double& res) {
+  const int lane = threadIdx.x & 31;
+  const double dead = walk_dead<KIND>();
+  const double none = KIND == K_DEC ? -2.0 : kFltMax;
+  const int R = KIND == K_DFD ? sh->pd.n1 : sh->pd.n1 - 1;
+  const int C = KIND == K_DFD ? sh->pd.n2 : sh->pd.n2 - 1;
+  const int nbr = (R + 31) >> 5, nbc = (C + 31) >> 5;
+  // (members past the last piece only keep the barriers)
+  const int pieces = walk_pieces(sh->pd, g.size, nbr, nbc);
+  const int m = g.rank;
+  const bool cut = w.cut0 >= 0 && pieces > 1;
+  const int i0 = min(cut ? w.cut0 : (int)((long long)nbr * min(m, pieces) / pieces), nbr);
+  const int i1 = cut && m + 1 < pieces ? min(w.cut1, nbr)
+                                       : (int)((long long)nbr * min(m + 1, pieces) / pieces);
+  WalkRecord* recs = reinterpret_cast<WalkRecord*>(sh->pd.recs);
+  if (lane == 0) {
+    sh->kind = KIND;
+    sh->flat = o.flat;
+    sh->level = level;
+    sh->rad = rad;
+  }
+  w.cur = 0;
+  w.n = 0;
+  w.blocks = 0;
+  w.rec_from = 0;
+  w.rec_end = -1;
+  double start = dead;
+  if (m == 0) {
+    if (KIND == K_DEC) start = 0.0;
+    if (KIND == K_VEFD && seed <= level) start = o.flat ? 0.0 : seed;
+    if (KIND == K_DFD) {
+      // the row below the grid: 0 at column 0
+      sh->up_v[0][0][lane] = lane == 0 ? 0.0 : dead;
+      if (lane == 0) sh->up_j[0][0] = 0;
+      w.n = 1;
+    }
+  }
+  __syncwarp();
+  res = none;
+  bool lost = false;
+  double c = 0.0;
+  if (pieces == 1) {
+    int rc = WALK_OK;
+    if (m == 0) rc = walk_rows<KIND>(wa, sh, w, 0, nbr, start, res, WALK_ALONE, nullptr, false, lost, c);
+    if (g.size == 1) return rc;
+    if (rc == WALK_ERROR) return rc;
+    if (m == 0 && lane == 0) {
+      WalkStat* q = g.stat[0] + g.first;
+      __stcg(&q->res, res);
+      __stcg(&q->gave_up, (int)(rc == WALK_GIVE_UP));
+    }
+    if (!walk_barrier(wa, g)) return WALK_ERROR;
+    const WalkStat* q = g.stat[0] + g.first;
+    res = __ldcg(&q->res);
+    return __ldcg(&q->gave_up) ? WALK_GIVE_UP : WALK_OK;
+  }
+  const bool on = m < pieces;
+  WalkStat me{0.0, none, 1, 0, 0, 0, 0, 0};
+  auto report = [&](int round) {
+    if (on && lane == 0) {
+      WalkStat* q = g.stat[round & 1] + g.first + m;
+      __stcg(&q->c, me.c);
+      __stcg(&q->res, me.res);
+      __stcg(&q->changed, me.changed);
+      __stcg(&q->which, me.which);
+      __stcg(&q->empty, me.empty);
+      __stcg(&q->part, me.part);
+      __stcg(&q->gave_up, me.gave_up);
+    }
+  };
+  int first_empty = 0;
+  double first_res = none;
+  if (on) {
+    bool err = false;
+    if (m > 0) err = !walk_start_row(wa, sh, w, i0, lost);
+    int rc = WALK_OK;
+    if (!err) rc = walk_rows<KIND>(wa, sh, w, i0, i1, start, me.res, WALK_RECORD, recs, m > 0, lost, c);
+    if (err || rc == WALK_ERROR) return WALK_ERROR;
+    if (rc == WALK_GIVE_UP) {
+      if (m == 0) me.gave_up = 1;
+      lost = true;  // (a start from too much: the piece is left to the rounds)
+      w.n = 0;
+      w.rec_end = -1;
+    }
+    walk_save_end(sh, w, g.end[0] + g.first + m);
+    first_empty = me.empty = w.n == 0 && i1 < nbr;
+    first_res = me.res;
+    me.part = lost;
+    if (KIND != K_DEC && w.rec_end >= 0) {
+      // the least value the piece ends with, in place of the constant in this report
+      double v = i1 == nbr ? me.res : dead;
+      for (int k = 0; k < w.n; ++k) v = fmin(v, sh->up_v[w.cur][k][lane]);
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) v = fmin(v, __shfl_xor_sync(kFull, v, s));
+      me.c = v < kFltMax ? v : 0.0;
+    }
+  }
+  report(0);
+  for (int round = 0;; ++round) {
+    if (!walk_barrier(wa, g)) return WALK_ERROR;
+    // the round's reports
+    const WalkStat* st = g.stat[round & 1] + g.first;
+    int moved = INT_MAX, bad = 0, hollow = INT_MAX, hollow_all = 0, part = 0;
+    double cc = 0.0;
+    for (int q = lane; q < pieces; q += 32) {
+      const WalkStat* s = st + q;
+      const int empty = __ldcg(&s->empty);
+      bad |= __ldcg(&s->gave_up);
+      if (round > 0 && __ldcg(&s->changed)) moved = min(moved, q);
+      if (empty) hollow = min(hollow, q);
+      const int lossy = __ldcg(&s->part);
+      part |= lossy;
+      if (empty && !lossy) hollow_all = 1;
+      cc = fmax(cc, __ldcg(&s->c));
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      moved = min(moved, __shfl_xor_sync(kFull, moved, d));
+      hollow = min(hollow, __shfl_xor_sync(kFull, hollow, d));
+      bad |= __shfl_xor_sync(kFull, bad, d);
+      hollow_all |= __shfl_xor_sync(kFull, hollow_all, d);
+      part |= __shfl_xor_sync(kFull, part, d);
+      cc = fmax(cc, __shfl_xor_sync(kFull, cc, d));
+    }
+    const double last = __ldcg(&st[pieces - 1].res);
+    int done = 0, rc = WALK_OK;
+    if (bad) {
+      done = 1;
+      rc = WALK_GIVE_UP;
+    } else if (round == 0) {
+      // a walk from everything that could be live died: so does the sweep
+      done = hollow_all || hollow == 0;
+      o.least = cc;
+      o.sure = !part;
+      me.c = 0.0;
+    } else if (moved == INT_MAX) {
+      // every piece was walked from its predecessor's end: the ends are the true ones
+      done = 1;
+      if (hollow == INT_MAX) res = (KIND == K_DEC || !(last < kFltMax)) ? last : fmax(cc, last);
+    } else {
+      done = hollow <= moved;  // (ends up to the first that moved are the true ones)
+    }
+    if (!done && round >= o.rounds) {
+      done = 1;
+      rc = WALK_UNSETTLED;
+    }
+    if (!done && round > 1 && ++w.rounds > o.limit) {
+      done = 1;
+      rc = WALK_GIVE_UP;
+    }
+    int from = 0, again = 0;
+    if (!done && on && m > 0) {
+      again = round == 0 || __ldcg(&st[m - 1].changed);
+      from = __ldcg(&st[m - 1].which);
+    }
+    if (done && rc == WALK_OK && res != none && on) {
+      walk_cut(w, recs, nbr, nbc, pieces, m);
+      o.band = true;
+    }
+    if (done) return rc;
+    const int was = me.which;
+    me.changed = 0;
+    if (again) {
+      walk_load_end(sh, w, g.end[from] + g.first + m - 1);
+      w.blocks = 0;
+      c = 0.0;
+      double r = none;
+      int q = WALK_OK;
+      if (w.n) q = walk_rows<KIND>(wa, sh, w, i0, i1, dead, r, WALK_AGAIN, recs, false, lost, c);
+      if (q == WALK_ERROR) return WALK_ERROR;
+      me.gave_up = q == WALK_GIVE_UP;
+      if (q == WALK_MET) {
+        me.which = 0;
+        me.c = c;
+        me.res = first_res;
+        me.empty = first_empty;
+        me.changed = was != 0;
+      } else {
+        me.which = was == 1 ? 2 : 1;
+        me.c = 0.0;
+        me.res = r;
+        me.empty = w.n == 0 && i1 < nbr;
+        me.changed = 1;
+        walk_save_end(sh, w, g.end[me.which] + g.first + m);
+      }
+    }
+    report(round + 1);
+  }
+}
+
+// The value of a min-max DP, by the group, or kFltMax if it exceeds the level (a WalkStatus is
+// returned).  Where the pieces' values do not meet their records within a few rounds (a wide band
+// keeps the values of its start apart, though its live columns soon agree), the least value a
+// path can have is guessed from the pieces' ends and settled by flat sweeps: some path survives
+// it, and none survives the next smaller number.
+template <int KIND>
+__device__ int walk_value(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup& g, double level,
+                          double seed, int limit, bool& band, double& res) {
+  constexpr int kRounds = 3;
+  int rc = WALK_OK;
+  // one sweep and the barrier after it; true when the caller goes on with `out`
+  double out = kFltMax;
+  WalkSweep o{false, kRounds, limit, 0.0, false, false};
+  auto sweep = [&](bool flat, int rounds, double at) -> bool {
+    o.flat = flat;
+    o.rounds = rounds;
+    rc = walk_sweep<KIND>(wa, sh, w, g, at, sqrt(at), seed, o, out);
+    band |= o.band;
+    if (!walk_barrier(wa, g)) rc = WALK_ERROR;
+    return rc == WALK_OK;
+  };
+  // flat sweeps around a candidate: 1 it is the value, 0 it is not, -1 error or given up
+  auto settles = [&](double x, bool sure) -> int {
+    if (!sweep(true, INT_MAX, x)) return -1;
+    if (!(out < kFltMax)) return 0;
+    if (sure || x == 0.0) return 1;
+    if (!sweep(true, INT_MAX, __longlong_as_double(__double_as_longlong(x) - 1))) return -1;
+    return out < kFltMax ? 0 : 1;
+  };
+  for (int turn = 0;; ++turn) {
+    if (sweep(false, turn < 2 ? kRounds : INT_MAX, level)) {
+      res = out;
+      return WALK_OK;
+    }
+    if (rc != WALK_UNSETTLED) return rc;
+    const double x = o.least;
+    const int s = settles(x, o.sure);
+    if (s < 0) return rc;
+    if (s == 1) {
+      res = x;
+      return WALK_OK;
+    }
+    // does any path survive the level?  (If so, the next turn's pieces start near it.)
+    if (!sweep(true, INT_MAX, level)) return rc;
+    if (!(out < kFltMax)) {
+      res = kFltMax;
+      return WALK_OK;
+    }
+  }
+}
+
+}  // namespace rfd
