@@ -805,7 +805,16 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
   __syncwarp();
   if (lane == 0) {
     PairDesc d = wa.pairs[p];
+    const int W = d.d == 2 ? RecW<2>::value : RecW<3>::value;
+    sh->seg_r = d.rowc;
+    sh->step_r = 1;
+    sh->seg_c = d.colrec + (W - 1);
+    sh->step_c = W;
     if (d.n1 < d.n2) {  // rows along the longer curve
+      sh->seg_r = sh->seg_c;
+      sh->step_r = W;
+      sh->seg_c = d.rowc;
+      sh->step_c = 1;
       const double* t = d.P;
       d.P = d.Q;
       d.Q = t;
@@ -953,7 +962,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) walk_kernel(WaveArgs wa, Walk
     return;
   }
   const int lane = threadIdx.x;
-  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, 0, -1, -1, -1, 0, -1, 0};
+  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, -1, -1, -1, 0, -1, 0};
   WalkGroup g;
   g.size = size;
   g.rank = blockIdx.x - group * size;
@@ -2585,8 +2594,12 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     const int search = nmem == 0 ? 4 : 0;
     // The DFD stays on the strips with the coarse bound, whose level opens most of the coarse
     // grid, and where the pairs outnumber the CTAs: the strips then run at the FP64 rate
-    // (5e11 cells/s), and the walk's few sweeps take as long.
-    const int dfd = ck || wcount[1] > 0 ? 0 : 1;
+    // (5e11 cells/s), and the walk's few sweeps take as long; and where a pair has one curve
+    // kWalkAspect times the other's length, whose DFD is large against the denser curve's spacing
+    // (2794 x 44 points: 7 ms of rounds against 1).
+    int dfd = ck || wcount[1] > 0 ? 0 : 1;
+    for (int64_t p = 0; p < npairs && dfd; ++p)
+      if (std::max(n1s[p], n2s[p]) >= kWalkAspect * std::min(n1s[p], n2s[p])) dfd = 0;
     if (!dfd && mode != MODE_DECIDE) {
       rc = strips(1);
       if (rc) return rc;

@@ -58,11 +58,9 @@ constexpr double kDecLive = 2.0;     // below: live
 // segment's A, 0.5/A and skip threshold.
 constexpr int kWalkPts = 33 * 3;
 constexpr int kWalkStage = 2 * kWalkPts + 6 * 32;
-// Values of a tile, in double2: listed edges' intervals (decision), or doubles, two to an
-// entry (VE-FD weights; the DFD's point distances of all 1024 cells).  Rows that no longer fit
-// are left to a second tile of the block.
-constexpr int kWalkVals = 640;
-constexpr int kWalkFitRows = kWalkVals / 64;  // rows that fit whatever they list
+// Values of a tile: every edge's interval (decision) or weight (VE-FD), or every cell's point
+// distance (DFD), in list order.
+constexpr int kWalkVals = 2048;
 
 // A block row's output list as recorded by the first walk of a piece (n < 0: too long to record),
 // and the chunks lo .. hi of the list as last walked.
@@ -80,10 +78,11 @@ struct WalkEnd {  // a piece's last list
 };
 // What a member reports at the end of a round: constant and result of its piece, whether its end
 // changed in the round, which copy of the end is current (0: the first walk's, 1 or 2), whether
-// it is empty; part: the first walk did not start from everything, or lost something on the way.
+// it is empty; part: the first walk did not start from everything, or lost something on the way;
+// skip: the piece has no rows (its members' neighbours are each other's).
 struct WalkStat {
   double c, res;
-  int changed, which, empty, part, gave_up, pad;
+  int changed, which, empty, part, gave_up, skip;
 };
 // Points 32 J .. 32 J + 32 of a curve within rad of the centre (rad infinite: no bound).
 struct WalkBall {
@@ -96,22 +95,28 @@ struct WalkShared {
   unsigned long long full[2];  // helpers -> propagator: tile ready
   unsigned long long req[2];   // propagator -> helpers: tile requested
   int req_i[2], req_j[2];      // block row (kStop: leave) and column
-  int req_r0[2], req_r1[2];    // rows of the block wanted
   int cancel[2];               // the speculative tile is not needed
-  int cnt[2], fit[2];          // edges listed; entries that are (see walk_tile)
-  int rows[2];                 // the tile holds rows req_r0 .. rows - 1
+  int cnt[2];                  // edges listed
+  int scan_to;                 // list a scan fills
   PairDesc pd;                 // the running sweep's grid
+  const double2 *seg_r, *seg_c;  // (|segment|^2, 0.5 / that) of the rows' and columns' segments,
+  int step_r, step_c;            // every step-th double2
   int kind, flat, filter, mat;
   double level, rad;           // pruning bound U or radius^2, and its root
   unsigned long long cells, cells64;
   uint4 mask[2][32];           // per row: listed right, listed top, live right, live top edges
+  uint4 risk[2][32];           // per row: right edges that end before 1, that start after 0, top
+                               // edges that end before 1
+  uint4 row_bits[32];          // per row of a block: columns reached, kept, passed, handing on
+  unsigned row_risk[32];       // ... kept from below at a value that may lie past the edge's end
   int2 base[2][32];            // per row: first right edge's and first top edge's value
   double bot[2][32];           // values rows enter / leave the block with
   int up_j[2][kWalkCap];       // live chunks of the row below / of the row being made
   double up_v[2][kWalkCap][32];
   double stage[2][kWalkStage];
   double2 vals[2][kWalkVals];
-  unsigned short list[2 * kWalkVals];
+  unsigned short list[kWalkVals];
+  double dead_row[32], spare_row[32];
   int nup, lost, scan_lo, scan_hi;  // scan of a piece's first row: chunks found, among which
 };
 constexpr size_t kWalkSmem = (sizeof(WalkShared) + 127) / 128 * 128;
@@ -124,28 +129,30 @@ __device__ __forceinline__ void walk_helper_sync() {
 
 // Skip threshold of the edges of a segment with squared length A: an edge whose far end point
 // lies farther than this (squared) from the other curve's point is certainly dead.  The point
-// is then more than rad + 0.005 (rad + length) from every point of the segment, a relative
+// is then more than rad + 0.004 (rad + length) from every point of the segment, a relative
 // margin of 1e-6 of the squared distances involved, while the FP64 code that computes the
 // edge errs by about 1e-8 of them (a discriminant at 0) and never calls such an edge live.
 // No skipping for degenerate segments (their free interval is [0, 1] at any radius), near the
 // ends of the exponent range, or where distances are lost in the coordinates' rounding.
+// (Lengths in FP32, rounded up, where they fit: an FP64 root is a third of the stage's time.)
 __device__ __forceinline__ double walk_threshold(double rad, double A, double mag) {
-  if (!(A > 1e-200)) return (double)INFINITY;
-  const double s = rad + sqrt(A);
+  const double len = A > 1e-30 && A < 1e30 ? 1.0005 * (double)sqrtf((float)A) : __dsqrt_rn(A);
+  const double s = rad + len;
   const double t = fmax(1.01 * s * s, 1e-14 * mag * mag);
-  return t < 1e200 ? t : (double)INFINITY;
+  return A > 1e-200 && t < 1e200 ? t : (double)INFINITY;
 }
 
-// Tile of block (bi, bj), rows [r0, r1), all helpers; tid in [0, 32 H).  A row whose edges no
-// longer fit ends the tile: rows[slot] is the first such row, and the entries listed before
-// its place (fit[slot]) are the valid ones.
-template <int D>
-__device__ void walk_tile(const PairDesc& pd, WalkShared* sh, int slot, int bi, int bj, int r0,
-                          int r1, int tid) {
+__device__ __forceinline__ void walk_prefetch(const void* p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
+// Tile of block (bi, bj), all helpers; tid in [0, 32 H).
+template <int D, int KIND>
+__device__ __forceinline__ void walk_tile(const PairDesc& pd, WalkShared* sh, int slot, int bi,
+                                          int bj, int tid) {
   const int lane = tid & 31, hw = tid >> 5;
   constexpr int NT = 32 * kWalkHelpers;
-  const int kind = sh->kind;
-  const bool dfd = kind == K_DFD;
+  constexpr bool dfd = KIND == K_DFD;
   double* P = sh->stage[slot];
   double* Q = P + kWalkPts;
   double* ra = Q + kWalkPts;  // row segments: A, 0.5/A, threshold
@@ -156,147 +163,137 @@ __device__ void walk_tile(const PairDesc& pd, WalkShared* sh, int slot, int bi, 
   double* cthr = cinv + 32;
   const int R = dfd ? pd.n1 : pd.n1 - 1, C = dfd ? pd.n2 : pd.n2 - 1;
   const int i0 = bi << 5, j0 = bj << 5;
-  const int nr = min(r1, R - i0), nc = min(32, C - j0);
+  const int nr = min(32, R - i0), nc = min(32, C - j0);
   {
     // points 32 bi .. 32 bi + 32 (clamped to the curve's end; clamped ones feed no cell)
-    const long long pe = (long long)pd.n1 * D, qe = (long long)pd.n2 * D;
-    for (int e = tid; e < 33 * D; e += NT) {
-      P[e] = __ldg(pd.P + min((long long)i0 * D + e, pe - 1));
-      Q[e] = __ldg(pd.Q + min((long long)j0 * D + e, qe - 1));
+    static_assert(33 * 3 <= NT, "one point coordinate a thread");
+    const long long pe = (long long)pd.n1 * D - 1, qe = (long long)pd.n2 * D - 1;
+    if (tid < 33 * D) {
+      P[tid] = __ldg(pd.P + min((long long)i0 * D + tid, pe));
+      Q[tid] = __ldg(pd.Q + min((long long)j0 * D + tid, qe));
+    }
+    // the points of the blocks right and up, which come next (16 doubles a line)
+    if (tid >= 192 && tid < 192 + 16) {
+      const int e = (tid - 192) * 16;
+      walk_prefetch(pd.P + min((long long)(i0 + 32) * D + e, pe));
+      walk_prefetch(pd.Q + min((long long)(j0 + 32) * D + e, qe));
     }
   }
-  if (tid < 32) {
-    sh->mask[slot][tid] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid == 0) {
-      sh->cnt[slot] = 0;
-      sh->fit[slot] = INT_MAX;
-      sh->rows[slot] = r1;
-    }
+  if (hw == 3) {
+    sh->mask[slot][lane] = make_uint4(0u, 0u, 0u, 0u);
+    if (KIND == K_DEC) sh->risk[slot][lane] = make_uint4(0u, 0u, 0u, 0u);
+    if (lane == 0) sh->cnt[slot] = 0;
   }
-  if (!dfd && hw >= kWalkHelpers - 2) {
-    // segment constants as prep_kernel forms them (|p - q|^2 does not depend on the order)
-    const bool col = hw == kWalkHelpers - 1;
-    const double* X = col ? pd.Q : pd.P;
-    const double* x = X + (size_t)min((col ? j0 : i0) + lane, (col ? C : R) - 1) * D;
-    double t[D], mag = 0.0;
+  if (!dfd && (hw == 4 || hw == 5)) {
+    // segment constants from prep_kernel's records
+    const bool col = hw == 5;
+    const int e = min((col ? j0 : i0) + lane, (col ? C : R) - 1);
+    const double2 rec = __ldg(col ? sh->seg_c + (size_t)e * sh->step_c : sh->seg_r + (size_t)e * sh->step_r);
+    const double* x = (col ? pd.Q : pd.P) + (size_t)(e + 1) * D;
+    double mag = 0.0;
 #pragma unroll
-    for (int k = 0; k < D; ++k) {
-      const double b = __ldg(x + D + k);
-      t[k] = __dsub_rn(b, __ldg(x + k));
-      mag = fmax(mag, fabs(b));
-    }
-    const double A = sq_sum<D>(t);
+    for (int k = 0; k < D; ++k) mag = fmax(mag, fabs(__ldg(x + k)));
     double* a = col ? ca : ra;
-    a[lane] = A;
-    a[32 + lane] = __ddiv_rn(0.5, A);
-    a[64 + lane] = walk_threshold(sh->rad, A, mag);
+    a[lane] = rec.x;
+    a[32 + lane] = rec.y;
+    a[64 + lane] = walk_threshold(sh->rad, rec.x, mag);
   }
   walk_helper_sync();
 
-  if (dfd) {
+  if constexpr (dfd) {
     // point distances are cheap: every cell
     double* W = reinterpret_cast<double*>(sh->vals[slot]);
     const double U = sh->level;
-    for (int r = r0 + hw; r < nr; r += kWalkHelpers) {
+    for (int r = hw; r < nr; r += kWalkHelpers) {
       const double w = dist_sq<D>(P + r * D, Q + lane * D);
       W[r * 32 + lane] = w;
-      const unsigned m = __ballot_sync(kFull, lane < nc && w <= U);
+      const unsigned m = __ballot_sync(kFull, (lane < nc) & (w <= U));
       if (lane == 0) sh->mask[slot][r].w = m;
     }
-    return;
-  }
-
-  // which edges can be live: lane = column
-  unsigned cells = 0, cells64 = 0;
-  const bool filt = kind == K_DEC && sh->filter;
-  const int cap = kind == K_DEC ? kWalkVals : 2 * kWalkVals;
-  {
-    double q[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) q[k] = Q[(lane + 1) * D + k];
-    const double ct = cthr[lane];
-    const unsigned lt = (1u << lane) - 1u;
-    // the warp's rows r0 + hw + 7 m together (independent tests), then one allocation for all
+  } else {
+    // which edges can be live: lane = column; the warp's rows hw + 7 m together (independent
+    // tests), then one allocation for all
     constexpr int M = (32 + kWalkHelpers - 1) / kWalkHelpers;
     unsigned br[M], bt[M];
     int n = 0;
+    {
+      double q[D];
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const int r = min(r0 + hw + m * kWalkHelpers, 31);
-      const bool in = lane < nc && r0 + hw + m * kWalkHelpers < nr;
-      const double s = dist_sq<D>(P + (r + 1) * D, q);
-      br[m] = __ballot_sync(kFull, in && (!(s > ct) || !(s < 1e200)));
-      bt[m] = __ballot_sync(kFull, in && (!(s > rthr[r]) || !(s < 1e200)));
-      n += __popc(br[m]) + __popc(bt[m]);
-      cells += __popc(br[m] | bt[m]);
+      for (int k = 0; k < D; ++k) q[k] = Q[(lane + 1) * D + k];
+      const double ct = cthr[lane];
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int r = min(hw + m * kWalkHelpers, 31);
+        const bool in = (lane < nc) & (hw + m * kWalkHelpers < nr);
+        const double s = dist_sq<D>(P + (r + 1) * D, q);
+        br[m] = __ballot_sync(kFull, in & !(s > ct));
+        bt[m] = __ballot_sync(kFull, in & !(s > rthr[r]));
+        n += __popc(br[m]) + __popc(bt[m]);
+      }
     }
     if (n) {
+      const unsigned lt = (1u << lane) - 1u;
       int at = 0;
       if (lane == 0) at = atomicAdd(&sh->cnt[slot], n);
       at = bcast(at);
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        const int r = r0 + hw + m * kWalkHelpers;
+        const int r = hw + m * kWalkHelpers;
         const int kr = __popc(br[m]), kt = __popc(bt[m]);
-        if (kr + kt == 0) continue;
-        if (at + kr + kt > cap) {
-          if (lane == 0) {
-            atomicMin(&sh->rows[slot], r);
-            atomicMin(&sh->fit[slot], at);
-          }
-        } else {
-          if (br[m] >> lane & 1u) sh->list[at + __popc(br[m] & lt)] = (unsigned short)(r << 5 | lane);
-          if (bt[m] >> lane & 1u)
-            sh->list[at + kr + __popc(bt[m] & lt)] = (unsigned short)(1024 | r << 5 | lane);
-          if (lane == 0) {
-            sh->mask[slot][r] = make_uint4(br[m], bt[m], 0u, 0u);
-            sh->base[slot][r] = make_int2(at, at + kr);
-          }
+        if (br[m] >> lane & 1u) sh->list[at + __popc(br[m] & lt)] = (unsigned short)(r << 5 | lane);
+        if (bt[m] >> lane & 1u)
+          sh->list[at + kr + __popc(bt[m] & lt)] = (unsigned short)(1024 | r << 5 | lane);
+        if ((lane == 0) & (kr + kt > 0)) {
+          sh->mask[slot][r] = make_uint4(br[m], bt[m], 0u, 0u);
+          sh->base[slot][r] = make_int2(at, at + kr);
         }
         at += kr + kt;
       }
     }
-  }
-  if (lane == 0 && cells) atomicAdd(&sh->cells, (unsigned long long)cells);
-  walk_helper_sync();
+    walk_helper_sync();
 
-  const int cnt = min(sh->cnt[slot], sh->fit[slot]);
-  const double level = sh->level;
-  const bool mat = sh->mat != 0;
-  if (*(volatile int*)&sh->cancel[slot]) return;
-  for (int k = tid; k < cnt; k += NT) {
-    const int e = sh->list[k], cell = e & 1023, r = cell >> 5, c = cell & 31;
-    const bool top = e >= 1024;
-    // right edge: p_{i+1} against q_j q_{j+1}; top edge: q_{j+1} against p_i p_{i+1}
-    const double* x = top ? Q + (c + 1) * D : P + (r + 1) * D;
-    const double* a = top ? P + r * D : Q + c * D;
-    double di[D];
+    const int cnt = sh->cnt[slot];
+    const double level = sh->level;
+    const bool mat = KIND == K_DEC && sh->mat != 0, filt = KIND == K_DEC && sh->filter != 0;
+    unsigned cells64 = 0;
+    if (*(volatile int*)&sh->cancel[slot]) return;
+    for (int k = tid; k < cnt; k += NT) {
+      const int e = sh->list[k], r = (e >> 5) & 31, c = e & 31;
+      const bool top = e >= 1024;
+      // right edge: p_{i+1} against q_j q_{j+1}; top edge: q_{j+1} against p_i p_{i+1}
+      const double* x = top ? Q + (c + 1) * D : P + (r + 1) * D;
+      const double* a = top ? P + r * D : Q + c * D;
+      double di[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) di[d] = __dsub_rn(a[D + d], a[d]);
-    const double A = top ? ra[r] : ca[c];
-    bool live;
-    if (kind == K_DEC) {
-      double lo, hi;
-      // the FP32 filter's certain answers need no FP64 (rfd_filter.h)
-      const int cls = filt ? interval_class32<D>(x, a, di, A, level) : 0;
-      if (cls == 0) {
-        free_interval<D>(x, a, di, A, top ? rinv[r] : cinv[c], level, lo, hi, mat);
-        if (filt) ++cells64;
+      for (int d = 0; d < D; ++d) di[d] = __dsub_rn(a[D + d], a[d]);
+      const double* seg = top ? ra + r : ca + c;
+      bool live;
+      if constexpr (KIND == K_DEC) {
+        double lo, hi;
+        // the FP32 filter's certain answers need no FP64 (rfd_filter.h)
+        const int cls = filt ? interval_class32<D>(x, a, di, seg[0], level) : 0;
+        if (cls == 0) {
+          free_interval<D>(x, a, di, seg[0], seg[32], level, lo, hi, mat);
+          cells64 += filt;
+        } else {
+          lo = cls == 1 ? -1.0 : 0.0;
+          hi = cls == 1 ? -2.0 : 1.0;
+        }
+        sh->vals[slot][k] = make_double2(lo, hi);
+        live = !(lo < 0.0);
+        uint4* risk = &sh->risk[slot][r];
+        if (live & (hi < 1.0)) atomicOr(top ? &risk->z : &risk->x, 1u << c);
+        if (live & !top & (lo > 0.0)) atomicOr(&risk->y, 1u << c);
       } else {
-        lo = cls == 1 ? -1.0 : 0.0;
-        hi = cls == 1 ? -2.0 : 1.0;
+        const double w = pt_seg_sq<D>(x, a, di, seg[0]);
+        reinterpret_cast<double*>(sh->vals[slot])[k] = w;
+        live = w <= level;
       }
-      sh->vals[slot][k] = make_double2(lo, hi);
-      live = !(lo < 0.0);
-    } else {
-      const double w = pt_seg_sq<D>(x, a, di, A);
-      reinterpret_cast<double*>(sh->vals[slot])[k] = w;
-      live = w <= level;
+      if (live) atomicOr(top ? &sh->mask[slot][r].w : &sh->mask[slot][r].z, 1u << c);
     }
-    if (live) atomicOr(top ? &sh->mask[slot][r].w : &sh->mask[slot][r].z, 1u << c);
+    // (edges; halved by the reader: at most the cells listed)
+    if (cells64) atomicAdd(&sh->cells64, (unsigned long long)cells64);
   }
-  // (edges, halved: at most the cells listed)
-  if (cells64) atomicAdd(&sh->cells64, (unsigned long long)cells64);
 }
 
 // Bounds of a curve's chunks (points 32 J - 1 .. 32 J + 32), one warp a chunk; a chunk with a
@@ -440,13 +437,20 @@ __device__ void walk_helpers(const WaveArgs& wa, WalkShared* sh) {
     if (!mbar_wait(&sh->req[slot], (seq >> 1) & 1, wa, clock64())) break;
     const int bi = *(volatile int*)&sh->req_i[slot], bj = *(volatile int*)&sh->req_j[slot];
     if (bi == kStop) break;
-    const int r0 = *(volatile int*)&sh->req_r0[slot], r1 = *(volatile int*)&sh->req_r1[slot];
     const PairDesc pd = sh->pd;
     if (bi == kScan) {
-      if (pd.d == 2) walk_scan<2>(pd, sh, r0, bj, tid);
-      else walk_scan<3>(pd, sh, r0, bj, tid);
-    } else if (pd.d == 2) walk_tile<2>(pd, sh, slot, bi, bj, r0, r1, tid);
-    else walk_tile<3>(pd, sh, slot, bi, bj, r0, r1, tid);
+      if (pd.d == 2) walk_scan<2>(pd, sh, sh->scan_to, bj, tid);
+      else walk_scan<3>(pd, sh, sh->scan_to, bj, tid);
+    } else if (sh->kind == K_DEC) {
+      if (pd.d == 2) walk_tile<2, K_DEC>(pd, sh, slot, bi, bj, tid);
+      else walk_tile<3, K_DEC>(pd, sh, slot, bi, bj, tid);
+    } else if (sh->kind == K_VEFD) {
+      if (pd.d == 2) walk_tile<2, K_VEFD>(pd, sh, slot, bi, bj, tid);
+      else walk_tile<3, K_VEFD>(pd, sh, slot, bi, bj, tid);
+    } else {
+      if (pd.d == 2) walk_tile<2, K_DFD>(pd, sh, slot, bi, bj, tid);
+      else walk_tile<3, K_DFD>(pd, sh, slot, bi, bj, tid);
+    }
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh->full[slot]);
     ++seq;
@@ -473,152 +477,331 @@ __device__ __forceinline__ bool walk_less(double a, double b) {
 __device__ __forceinline__ double walk_min(double a, double b) { return walk_less(a, b) ? a : b; }
 __device__ __forceinline__ double walk_max(double a, double b) { return walk_less(a, b) ? b : a; }
 
-// One row's tile words for this lane's column, in the two dependent steps they load in: the
-// row's masks and places, then the values and (decision) what the left neighbour would pass on.
-struct WalkHead {
-  uint4 m;
-  int2 base;
-};
-struct WalkRow {
-  unsigned mr, mt;  // live right / top edges of the row
-  double2 r, t;     // their values (VE-FD: weights in .x; DFD: t.x)
-};
-template <int KIND>
-__device__ __forceinline__ WalkHead walk_row_head(const WalkShared* sh, int slot, int r) {
-  WalkHead h;
-  h.m = sh->mask[slot][r];
-  if (KIND != K_DFD) h.base = sh->base[slot][r];
-  return h;
-}
-template <int KIND>
-__device__ __forceinline__ WalkRow walk_row_load(const WalkShared* sh, int slot, int r,
-                                                 const WalkHead& h, bool flat) {
-  const int lane = threadIdx.x & 31;
-  WalkRow w;
-  w.mr = h.m.z;
-  w.mt = h.m.w;
-  if (KIND == K_DFD) {
-    const double t = reinterpret_cast<const double*>(sh->vals[slot])[r * 32 + lane];
-    w.t.x = flat ? 0.0 : t;
-  } else {
-    // (a lane without a listed edge reads another's value and does not use it; the places of a
-    // row that lists nothing are stale, hence the bound)
-    const unsigned lt = (1u << lane) - 1u;
-    constexpr unsigned cap = (KIND == K_DEC ? kWalkVals : 2 * kWalkVals) - 1;
-    const unsigned kr = min((unsigned)h.base.x + __popc(h.m.x & lt), cap);
-    const unsigned kt = min((unsigned)h.base.y + __popc(h.m.y & lt), cap);
-    if (KIND == K_DEC) {
-      w.r = sh->vals[slot][kr];
-      w.t = sh->vals[slot][kt];
-    } else {
-      const double a = reinterpret_cast<const double*>(sh->vals[slot])[kr];
-      const double b = reinterpret_cast<const double*>(sh->vals[slot])[kt];
-      w.r.x = flat ? 0.0 : a;
-      w.t.x = flat ? 0.0 : b;
-    }
-  }
-  return w;
-}
-// Decision: the value the column to the left passes on when it is live from below (lane 0: the
-// value the row enters with), and the columns whose top edge ends before it.
-struct WalkPrev {
-  double v;
-  unsigned late;
-};
-__device__ __forceinline__ WalkPrev walk_row_prev(const WalkRow& w, double x0) {
-  WalkPrev p;
-  p.v = __shfl_up_sync(kFull, w.t.x, 1);
-  p.v = (threadIdx.x & 31) == 0 ? x0 : p.v;
-  p.late = __ballot_sync(kFull, __double_as_longlong(w.t.y) < __double_as_longlong(p.v));
-  return p;
+// Place of a listed edge's value: the row's first one and the listed edges left of column c.  (A
+// column without a listed edge, or a row that lists none and whose place is stale, gives some
+// place within the tile; its value is not used.)
+__device__ __forceinline__ unsigned walk_place(int first, unsigned listed, int c) {
+  return min((unsigned)first + __popc(listed & ((1u << c) - 1u)), (unsigned)kWalkVals - 1u);
 }
 
-// One row of a block (lane = column).  F: value handed up by the row below, replaced by this
-// row's; V: its live columns.  in: whether the row enters the block live, with value x0.  y:
-// value this lane's column hands to the right; Y: the columns that hand on a live one.
-//
-// Decision.  The value runs right through top edges: column j hands on t.lo when it is live
-// from below, else max(t.lo, x) if the incoming x is at most t.hi.  Whether a value arrives is
-// a carry chain of bits (generate: live from below and the edge free; propagate: edge free),
-// one addition for the row - exact unless a value that passed a column without support from
-// below meets an edge that ends before it.  The value such a pass brings is the previous
-// column's t.lo when the pass is one column long, so one comparison settles those; longer
-// passes, and comparisons that fail, go column by column (the band is a few cells wide: rare).
-template <int KIND>
-__device__ __forceinline__ void walk_row(const WalkRow& w, const WalkPrev& pv, bool in, double x0,
+// Row r of a block's decision, every value formed (lane = column).  F: value handed up by the row
+// below, replaced by this row's; V: its live columns.  in: whether the row enters the block
+// live, with value x0.  y: value this lane's column hands to the right; Y: the columns that
+// hand on a live one.  The value runs right through top edges: column j hands on t.lo when it
+// is live from below, else max(t.lo, x) if the incoming x is at most t.hi; repeated until no
+// column changes (as often as the longest run of columns without support from below).
+__device__ __forceinline__ void walk_row(const WalkShared* sh, int slot, int r, bool in, double x0,
                                          double& F, unsigned& V, double& y, unsigned& Y) {
   const int lane = threadIdx.x & 31;
   const unsigned bit = 1u << lane;
-  const double dead = walk_dead<KIND>();
-  const bool br = (w.mr & bit) != 0u, bt = (w.mt & bit) != 0u;
-  const double first = in ? x0 : dead;  // what enters column 0
-  if (KIND == K_DEC) {
-    const unsigned gen = V & w.mt;
-    unsigned X = (w.mt + gen + (unsigned)in) ^ w.mt ^ gen;  // live values arriving at a column
-    const unsigned pass = X & ~V & w.mt;
-    const bool up = (V & bit) != 0u;
-    const bool reset = up | !walk_less(w.t.x, pv.v);
-    y = reset ? w.t.x : pv.v;
-    Y = w.mt & (V | X);
-    if (pass & (pv.late | (pass << 1))) {
-      double x;
-      y = bt & up ? w.t.x : dead;
-      for (;;) {
-        x = __shfl_up_sync(kFull, y, 1);
-        x = lane == 0 ? first : x;
-        const bool ends = !bt | (!up & walk_less(w.t.y, x));
-        const bool own = up | !walk_less(w.t.x, x);
-        double yn = own ? w.t.x : x;
-        yn = ends ? dead : yn;
-        const bool moved = walk_less(yn, y) | walk_less(y, yn);
-        y = yn;
-        if (!__any_sync(kFull, moved)) break;
-      }
-      X = __ballot_sync(kFull, walk_live<KIND>(x));
-      Y = __ballot_sync(kFull, walk_live<KIND>(y));
-    }
-    const bool xl = (X & bit) != 0u;
-    const bool ok = br & (xl | !walk_less(w.r.y, F));
-    const bool own = xl | !walk_less(w.r.x, F);
-    const double f = own ? w.r.x : F;
-    F = ok ? f : dead;
-    V = __ballot_sync(kFull, ok);
-  } else {
-    // y_j = max(w_j, min(F_j, y_{j-1})): from the values entering from below, repeated while a
-    // changed column has a live right neighbour (as often as the longest run of cells reached
-    // from the left)
-    double x = lane == 0 ? first : dead;
-    y = walk_max(w.t.x, walk_min(F, x));
-    y = bt ? y : dead;
-    for (;;) {
-      x = __shfl_up_sync(kFull, y, 1);
-      x = lane == 0 ? first : x;
-      double yn = walk_max(w.t.x, walk_min(F, x));
-      yn = bt ? yn : dead;
-      const unsigned moved = __ballot_sync(kFull, walk_less(yn, y));
-      y = yn;
-      if ((moved << 1) & w.mt) continue;
-      if (moved) {
-        x = __shfl_up_sync(kFull, y, 1);
-        x = lane == 0 ? first : x;
-      }
-      break;
-    }
-    if (KIND == K_DFD) {
-      F = walk_min(y, x);
-    } else {
-      const double f = walk_max(w.r.x, walk_min(F, x));
-      F = br ? f : dead;
-    }
-    V = __ballot_sync(kFull, walk_live<KIND>(F));
-    Y = __ballot_sync(kFull, walk_live<KIND>(y));
+  const uint4 m = sh->mask[slot][r];
+  const int2 base = sh->base[slot][r];
+  const double2 er = sh->vals[slot][walk_place(base.x, m.x, lane)];
+  const double2 et = sh->vals[slot][walk_place(base.y, m.y, lane)];
+  const bool br = (m.z & bit) != 0u, bt = (m.w & bit) != 0u, up = (V & bit) != 0u;
+  const double first = in ? x0 : kDecDead;  // what enters column 0
+  double x;
+  y = bt & up ? et.x : kDecDead;
+  for (;;) {
+    x = __shfl_up_sync(kFull, y, 1);
+    x = lane == 0 ? first : x;
+    const bool ends = !bt | (!up & walk_less(et.y, x));
+    const bool own = up | !walk_less(et.x, x);
+    double yn = own ? et.x : x;
+    yn = ends ? kDecDead : yn;
+    const bool moved = walk_less(yn, y) | walk_less(y, yn);
+    y = yn;
+    if (!__any_sync(kFull, moved)) break;
   }
+  const bool xl = walk_live<K_DEC>(x);
+  const bool ok = br & (xl | !walk_less(er.y, F));
+  const bool own = xl | !walk_less(er.x, F);
+  const double f = own ? er.x : F;
+  F = ok ? f : kDecDead;
+  V = __ballot_sync(kFull, ok);
+  Y = __ballot_sync(kFull, walk_live<K_DEC>(y));
+}
+
+// Rows r .. nr - 1 of a block as far as bits settle them (decision and flat sweeps).  First the
+// live columns, row by row, as if no value stood in the way of another: whether a value arrives
+// at a column is a carry chain (generate: live from below and the top edge free; propagate: top
+// edge free), one addition for the row's 32 columns.  A value can stand in the way only where
+// an edge that ends before 1 is kept from below by a value above 0, or passed without support
+// from below; bits say where that may be (few places in a thin band), and there the values are
+// formed and compared, lane = row.  The values handed on are formed last, a column of the last
+// row from its run of rows.
+// Returns nr, or the first row where a value does meet an edge that ends before it: what is handed
+// on is then as of the row before.
+template <int KIND>
+__device__ __forceinline__ int walk_bits(WalkShared* sh, int slot, int r, int nr, unsigned bmask,
+                                         const double* bin, double* bout, double& F, unsigned& V,
+                                         unsigned& omask, unsigned& Y) {
+  const int lane = threadIdx.x & 31;
+  const unsigned bit = 1u << lane;
+  const double dead = walk_dead<KIND>();
+  // from the first row that has something live to the last (a loop of few instructions: code that
+  // runs once a block is fetched at 5 cycles an instruction)
+  const unsigned entries = bmask & (0xffffffffu << r);
+  const int r0 = V ? r : __ffs(entries) - 1;
+  int r1 = r0;
+  unsigned v = V, yl = 0u;
+  {
+    unsigned above = KIND == K_DEC ? __ballot_sync(kFull, walk_live<KIND>(F) & (F > 0.0)) : 0u;
+    unsigned in = entries >> r0;
+    uint2 m = *reinterpret_cast<const uint2*>(&sh->mask[slot][r0].z), k = make_uint2(0u, 0u);
+    if (KIND == K_DEC) k = *reinterpret_cast<const uint2*>(&sh->risk[slot][r0].x);
+#pragma unroll 2
+    do {
+      const int rn = min(r1 + 1, 31);
+      const uint2 mn = *reinterpret_cast<const uint2*>(&sh->mask[slot][rn].z);
+      uint2 kn = k;
+      if (KIND == K_DEC) kn = *reinterpret_cast<const uint2*>(&sh->risk[slot][rn].x);
+      const unsigned gen = v & m.y;
+      const unsigned X = (m.y + gen + (in & 1u)) ^ m.y ^ gen;  // live values arriving
+      const unsigned any = X | v;
+      yl = m.y & any;
+      const unsigned ok = KIND == K_DFD ? (yl | X) : m.x & any;
+      sh->row_bits[r1] = make_uint4(X, ok, X & ~v & m.y, yl);
+      if (KIND == K_DEC) {
+        const unsigned held = above & ~X;  // columns kept from below, at values that may exceed 0
+        sh->row_risk[r1] = ok & held & k.x;
+        above = ok & (k.y | held);
+      }
+      v = ok;
+      m = mn;
+      k = kn;
+      in >>= 1;
+      ++r1;
+    } while ((r1 < nr) & ((v | in) != 0u));
+  }
+  __syncwarp();
+  const bool mine = (lane >= r0) & (lane < r1);
+  uint4 rb = sh->row_bits[lane];
+  if (!mine) rb = make_uint4(0u, 0u, 0u, 0u);
+  unsigned top = r1 == nr ? v : 0u;
+  unsigned out = __ballot_sync(kFull, (rb.w >> 31) != 0u);
+  if (KIND != K_DEC) {
+    if (rb.w >> 31) bout[lane] = 0.0;
+    F = top & bit ? 0.0 : dead;
+  } else {
+    const uint4 m = sh->mask[slot][lane];
+    const int2 base = sh->base[slot][lane];
+    const double2* vals = sh->vals[slot];
+    bool clash = false;
+    // passes, left to right, in the rows where one meets an edge that ends before 1 or is the
+    // last column's
+    unsigned todo = rb.z & (sh->risk[slot][lane].z | 0x80000000u) ? rb.z : 0u;
+    double x = 0.0;
+    int before = -2;  // column passed last, x what it handed on
+    unsigned rows = __ballot_sync(kFull, todo != 0u);
+    if ((int)__reduce_max_sync(kFull, __popc(todo)) > 1 + __popc(rows)) {
+      // few rows with long passes: these one by one, lane = column, the largest start of a pass so
+      // far by a scan over the columns (about what two steps of the loop below take)
+      for (; rows; rows &= rows - 1u) {
+        const int q = __ffs(rows) - 1;
+        const uint4 b = sh->row_bits[q], mq = sh->mask[slot][q];
+        const double2 t = vals[walk_place(sh->base[slot][q].y, mq.y, lane)];
+        const bool pass = (b.z & bit) != 0u;
+        double g = (lane == 0) & pass ? walk_max(t.x, bin[q]) : t.x;
+        const unsigned heads = ~b.z | 1u;
+        const int run = lane - (31 - __clz(heads & (bit | (bit - 1u))));
+#pragma unroll 1
+        for (int d = 1; d < 32; d <<= 1) {
+          const double h = __shfl_up_sync(kFull, g, d);
+          g = run >= d ? walk_max(g, h) : g;
+        }
+        double from = __shfl_up_sync(kFull, g, 1);
+        from = lane == 0 ? bin[q] : from;
+        const bool hits = __any_sync(kFull, pass & walk_less(t.y, from));
+        const double end = __shfl_sync(kFull, g, 31);
+        clash |= (lane == q) & hits;
+        x = lane == q ? end : x;
+        before = (lane == q) & (int)(b.z >> 31) ? 31 : before;
+      }
+      todo = 0u;
+    }
+    while (__any_sync(kFull, todo != 0u)) {
+      const int c = todo ? __ffs(todo) - 1 : 0;
+      const double own = c == 0 ? bin[lane] : vals[walk_place(base.y, m.y, c - 1)].x;
+      const double2 t = vals[walk_place(base.y, m.y, c)];
+      const double from = before == c - 1 ? x : own;
+      clash |= (todo != 0u) & walk_less(t.y, from);
+      x = todo ? walk_max(t.x, from) : x;
+      before = todo ? c : before;
+      todo &= todo - 1u;
+    }
+    if (rb.w >> 31) bout[lane] = before == 31 ? x : vals[walk_place(base.y, m.y, 31)].x;
+    // values kept from below that may lie past the edge's end: down the column to where the run
+    // started, the largest start on the way
+    todo = mine ? sh->row_risk[lane] : 0u;
+    int row = lane;  // row looked at last, of the run under cell (lane, lowest bit of todo)
+    double f = 0.0;
+    unsigned cols = __reduce_or_sync(kFull, todo);
+    if (cols && __popc(cols) <= 2) {
+      // one or two columns: each by a scan over its rows
+      for (; cols; cols &= cols - 1u) {
+        const int c = __ffs(cols) - 1;
+        const double2 e = vals[walk_place(base.x, m.x, c)];
+        const bool reached = (rb.x >> c & 1u) != 0u;
+        const double f0 = __shfl_sync(kFull, F, c);
+        const bool below = (lane == r0) & !reached;
+        double g = below ? walk_max(e.x, f0) : e.x;
+        const unsigned heads = __ballot_sync(kFull, reached | (lane <= r0) | !(rb.y >> c & 1u));
+        const int run = lane - (31 - __clz(heads & (bit | (bit - 1u))));
+#pragma unroll 1
+        for (int d = 1; d < 32; d <<= 1) {
+          const double h = __shfl_up_sync(kFull, g, d);
+          g = run >= d ? walk_max(g, h) : g;
+        }
+        double under = __shfl_up_sync(kFull, g, 1);
+        under = below ? f0 : under;
+        clash |= ((todo >> c & 1u) != 0u) & walk_less(e.y, under);
+      }
+      todo = 0u;
+    }
+    while (__any_sync(kFull, todo != 0u)) {
+      const int c = todo ? __ffs(todo) - 1 : 0;
+      const double f0 = __shfl_sync(kFull, F, c);
+      row = max(row - 1, r0 - 1);
+      const int q = max(row, r0);
+      const double lo = vals[walk_place(sh->base[slot][q].x, sh->mask[slot][q].x, c)].x;
+      f = walk_max(f, row < r0 ? f0 : lo);
+      const bool start = (row < r0) | ((sh->row_bits[q].x >> c & 1u) != 0u);
+      const double hi = vals[walk_place(base.x, m.x, c)].y;
+      clash |= (todo != 0u) & start & walk_less(hi, f);
+      todo = start ? todo & (todo - 1u) : todo;
+      row = start ? lane : row;
+      f = start ? 0.0 : f;
+    }
+    const unsigned bad = __ballot_sync(kFull, clash);
+    if (bad) {
+      // up to there
+      nr = __ffs(bad) - 1;
+      if (nr == r0) return nr;
+      r1 = nr;
+      const uint4 b = sh->row_bits[nr - 1];
+      top = b.y;
+      yl = b.w;
+      out &= (1u << nr) - 1u;
+    }
+    // the last row's values
+    double Fn = dead;
+    for (unsigned cols = top; cols; cols &= cols - 1u) {
+      const int c = __ffs(cols) - 1;
+      const bool reached = (rb.x >> c & 1u) != 0u;
+      const bool below = (lane == r0) & !reached;  // the run starts in the row below
+      const double lo = vals[walk_place(base.x, m.x, c)].x, f0 = __shfl_sync(kFull, F, c);
+      const unsigned heads = __ballot_sync(kFull, reached | (lane == r0) | !(rb.y >> c & 1u));
+      const int head = 31 - __clz(heads & (nr == 32 ? kFull : (1u << nr) - 1u));
+      // (rows head .. nr - 1 are the run; others take no part)
+      double g = (lane >= head) & (lane < nr) ? lo : 0.0;
+      g = (lane == head) & below ? walk_max(g, f0) : g;
+#pragma unroll 1
+      for (int d = 16; d > 0; d >>= 1) g = walk_max(g, __shfl_xor_sync(kFull, g, d));
+      Fn = lane == c ? g : Fn;
+    }
+    F = Fn;
+  }
+  V = top;
+  omask |= out;
+  Y = r1 == nr ? yl : 0u;
+  __syncwarp();
+  return nr;
+}
+
+// A block of a min-max sweep with its values: a skewed sweep (lane = row, step t: column t -
+// lane) over the anti-diagonals that have a live value.  upv / V: the row below (values, live
+// columns); rows enter with bin where bmask says so and leave with bout; out: the row handed on.
+// y, f: last column's and row's values of this lane's row.
+template <int KIND>
+__device__ __forceinline__ void walk_values(const WalkShared* sh, int slot, int nr, int nc,
+                                            const double* upv, unsigned V, unsigned bmask,
+                                            const double* bin, double* bout, unsigned& omask,
+                                            double* out, double& y, double& f) {
+  const int lane = threadIdx.x & 31;
+  const double dead = kFltMax;
+  const double* vals = reinterpret_cast<const double*>(sh->vals[slot]);
+  const uint4 m = sh->mask[slot][lane];
+  int kr = 0, kt = lane * 32;
+  if (KIND == K_VEFD) {
+    const int2 base = sh->base[slot][lane];
+    kr = max(min(base.x, kWalkVals), 0);  // (stale where the row lists nothing)
+    kt = max(min(base.y, kWalkVals), 0);
+  }
+  double bot = bmask >> lane & 1u ? bin[lane] : dead, carry = dead;
+  out[lane] = dead;
+  __syncwarp();
+  const bool store = lane == nr - 1;
+  int t = min(V ? __ffs(V) - 1 : 64, bmask ? __ffs(bmask) - 1 : 64);
+  // (columns skipped at the start: their listed edges too)
+  auto skip = [&](int c) {
+    if (KIND == K_VEFD && c > 0) {
+      const unsigned below = c > 31 ? kFull : (1u << c) - 1u;
+      kr += __popc(m.x & below);
+      kt += __popc(m.y & below);
+    }
+  };
+  skip(t - lane);
+  while (t < nr + nc - 1) {
+#pragma unroll 2
+    for (int u = 0; u < 4; ++u, ++t) {
+      const int c = t - lane;
+      const bool act = (unsigned)c < (unsigned)nc;
+      const unsigned bit = act ? 1u << c : 0u;
+      double left = __shfl_up_sync(kFull, carry, 1);
+      const double low = upv[t & 31];
+      left = lane == 0 ? low : left;
+      const double in = walk_min(left, bot);
+      double ncarry, nbot;
+      if (KIND == K_VEFD) {
+        const double wr = vals[kr], wt = vals[kt];
+        kr += (m.x & bit) != 0u;
+        kt += (m.y & bit) != 0u;
+        ncarry = walk_max(wr, in);
+        ncarry = (m.z & bit) != 0u ? ncarry : dead;
+        nbot = walk_max(wt, in);
+        nbot = (m.w & bit) != 0u ? nbot : dead;
+      } else {
+        const double w = vals[kt + max(min(c, 31), 0)];
+        nbot = walk_max(w, in);
+        nbot = (m.w & bit) != 0u ? nbot : dead;
+        ncarry = walk_min(nbot, bot);
+      }
+      carry = act ? ncarry : carry;
+      bot = act ? nbot : bot;
+      if (act & store) out[c] = carry;
+    }
+    // rows at work in step t, or handing a live value to one that is
+    const bool busy = ((lane <= t) & (lane + 31 >= t) & (bot < dead)) |
+                      ((lane < t) & (lane + 32 >= t) & (lane < 31) & (carry < dead));
+    if (!__any_sync(kFull, busy)) {
+      // all dead: on to the next live input, if any
+      const unsigned fb = __ballot_sync(kFull, (lane > t) & (bot < dead));
+      const unsigned fu = t < 32 ? V & (0xffffffffu << t) : 0u;
+      if (!(fb | fu)) break;
+      const int to = __ffs(fb | fu) - 1;
+      if (KIND == K_VEFD) {
+        // listed edges of the columns jumped over
+        const int c0 = min(max(t - lane, 0), 32), c1 = min(max(to - lane, 0), 32);
+        const unsigned b1 = c1 > 31 ? kFull : (1u << c1) - 1u, b0 = c0 > 31 ? kFull : (1u << c0) - 1u;
+        kr += __popc(m.x & b1 & ~b0);
+        kt += __popc(m.y & b1 & ~b0);
+      }
+      t = to;
+    }
+  }
+  __syncwarp();
+  omask = __ballot_sync(kFull, (bot < dead) & (lane < nr));
+  if (lane < nr) bout[lane] = bot;
+  y = bot;
+  f = carry;
+  __syncwarp();
 }
 
 // Walk of one CTA: requests outstanding, and the list of the row below.
 struct Walk {
   unsigned seq_p, seq_c;  // tiles requested, taken
-  int pi, pj, pr;         // the outstanding request (pi < 0: none)
+  int pi, pj;             // the outstanding request (pi < 0: none)
   int cur, n;             // list of the row below: buffer and live chunks
   long long blocks;       // blocks swept
   int rec_from, rec_end;  // block rows whose records this sweep can be met at
@@ -634,14 +817,11 @@ enum WalkStatus : int { WALK_OK = 0, WALK_ERROR, WALK_GIVE_UP, WALK_MET, WALK_UN
 // from the true start, recording every block row's list; again, until it meets a record.
 enum WalkMode : int { WALK_ALONE = 0, WALK_RECORD = 1, WALK_AGAIN = 2 };
 
-__device__ __forceinline__ void walk_request(WalkShared* sh, Walk& w, int i, int j, int r0 = 0,
-                                             int r1 = 32) {
+__device__ __forceinline__ void walk_request(WalkShared* sh, Walk& w, int i, int j) {
   if ((threadIdx.x & 31) == 0) {
     const int slot = w.seq_p & 1;
     *(volatile int*)&sh->req_i[slot] = i;
     *(volatile int*)&sh->req_j[slot] = j;
-    *(volatile int*)&sh->req_r0[slot] = r0;
-    *(volatile int*)&sh->req_r1[slot] = r1;
     *(volatile int*)&sh->cancel[slot] = 0;
     mbar_arrive(&sh->req[slot]);
   }
@@ -649,7 +829,6 @@ __device__ __forceinline__ void walk_request(WalkShared* sh, Walk& w, int i, int
   ++w.seq_p;
   w.pi = i;
   w.pj = j;
-  w.pr = r0;
 }
 // The propagator's wait for a tile (bounded).  It polls: the helpers' waits suspend
 // (mbarrier.try_wait), but this one is on the sweep's chain.
@@ -688,12 +867,11 @@ __device__ __forceinline__ bool walk_drop(const WaveArgs& wa, WalkShared* sh, Wa
   __syncwarp();
   return walk_take(wa, sh, w) >= 0;
 }
-// The tile of block (i, j) from row r0 on: taken if it is the outstanding request.
-__device__ __forceinline__ int walk_get(const WaveArgs& wa, WalkShared* sh, Walk& w, int i, int j,
-                                        int r0, int r1 = 32) {
-  if (w.pi != i || w.pj != j || w.pr != r0) {
+// The tile of block (i, j): taken if it is the outstanding request.
+__device__ __forceinline__ int walk_get(const WaveArgs& wa, WalkShared* sh, Walk& w, int i, int j) {
+  if ((w.pi != i) | (w.pj != j)) {
     if (!walk_drop(wa, sh, w)) return -1;
-    walk_request(sh, w, i, j, r0, r1);
+    walk_request(sh, w, i, j);
   }
   return walk_take(wa, sh, w);
 }
@@ -714,6 +892,7 @@ __device__ int walk_rows(const WaveArgs& wa, WalkShared* sh, Walk& w, int i0, in
   const int nbr = (R + 31) >> 5, nbc = (C + 31) >> 5;
   const bool flat = KIND != K_DEC && sh->flat;
   int j_min = INT_MAX, j_max = 0;
+  unsigned cells = 0;
   int status = WALK_OK;
   for (int i = i0; i < i1 && status == WALK_OK; ++i) {
     const int in = w.cur, ob = w.cur ^ 1;
@@ -743,10 +922,11 @@ __device__ int walk_rows(const WaveArgs& wa, WalkShared* sh, Walk& w, int i0, in
         j = sh->up_j[in][k];
       }
       const bool have = k < w.n && sh->up_j[in][k] == j;
-      double F = have ? sh->up_v[in][k][lane] : dead;
+      const double* upv = have ? sh->up_v[in][k] : sh->dead_row;
+      double F = upv[lane];
       unsigned V = __ballot_sync(kFull, walk_live<KIND>(F));
       k += have;
-      int slot = walk_get(wa, sh, w, i, j, 0);
+      const int slot = walk_get(wa, sh, w, i, j);
       if (slot < 0) { status = WALK_ERROR; break; }
       // effort against progress: a thin band lists a few hundred edges a block and goes from block
       // to block right or up
@@ -757,84 +937,76 @@ __device__ int walk_rows(const WaveArgs& wa, WalkShared* sh, Walk& w, int i0, in
         status = WALK_GIVE_UP;
         break;
       }
-      int rows = *(volatile int*)&sh->rows[slot];
       {
         // the next block: right when this one's last column has a live edge, else the next
         // chunk of the row, else up
         const uint4 m = sh->mask[slot][lane];
         const bool right = __any_sync(kFull, m.w >> 31);
+        cells += __reduce_add_sync(kFull, __popc(m.x | m.y));
         const bool more = k < w.n;
+        const int jn = more ? sh->up_j[in][k] : 0;
         int ni = -1, nj = 0;
-        if (rows < nr) {
-          // (this block's other rows come first)
-        } else if (j + 1 < nbc && (right || (more && sh->up_j[in][k] == j + 1))) {
+        if (j + 1 < nbc && (right | (more & (jn == j + 1)))) {
           ni = i;
           nj = j + 1;
         } else if (more) {
           ni = i;
-          nj = sh->up_j[in][k];
+          nj = jn;
         } else if (i + 1 < i1) {
           ni = i + 1;
           nj = on ? sh->up_j[ob][0] : j;
         }
         if (ni >= 0) walk_request(sh, w, ni, nj);
       }
-      const bool last = i == nbr - 1 && j == nbc - 1;
-      unsigned omask = 0u;
+      unsigned omask = 0u, Y = 0u;
       const double* bin = sh->bot[bb];
       double* bout = sh->bot[bb ^ 1];
-      int r = 0;
-      while (true) {
-        if (V == 0u) {
-          // nothing from below: on to the next row that enters live, if any
-          const unsigned left = r < 32 ? bmask & (0xffffffffu << r) : 0u;
-          if (!left) { r = nr; break; }
-          r = __ffs(left) - 1;
-        }
-        if (r >= nr) break;
-        if (r >= rows) {
-          slot = walk_get(wa, sh, w, i, j, r);
-          if (slot >= 0 && *(volatile int*)&sh->rows[slot] <= r)
-            slot = walk_get(wa, sh, w, i, j, r, min(32, r + kWalkFitRows));
-          if (slot < 0) { status = WALK_ERROR; break; }
-          rows = *(volatile int*)&sh->rows[slot];
-        }
-        // rows r .. stop - 1, their loads two and one rows ahead
-        const int stop = min(rows, nr);
-        auto enter = [&](int q) { return bin[min(q, 31)]; };
-        WalkRow cur = walk_row_load<KIND>(sh, slot, r, walk_row_head<KIND>(sh, slot, r), flat);
-        WalkHead head = walk_row_head<KIND>(sh, slot, min(r + 1, 31));
-        double x0 = enter(r);
-        WalkPrev pv;
-        if (KIND == K_DEC) pv = walk_row_prev(cur, x0);
-        double y;
-        unsigned Y;
-        WalkRow at;
-        do {
-          const WalkRow nxt = walk_row_load<KIND>(sh, slot, min(r + 1, 31), head, flat);
-          head = walk_row_head<KIND>(sh, slot, min(r + 2, 31));
-          const double x1 = enter(r + 1);
-          walk_row<KIND>(cur, pv, (bmask >> r) & 1u, x0, F, V, y, Y);
-          if ((lane == 31) & (int)(Y >> 31)) bout[r] = y;
-          omask |= (Y >> 31) << r;
-          if (KIND == K_DEC) pv = walk_row_prev(nxt, x1);
-          at = cur;
-          cur = nxt;
-          x0 = x1;
-          ++r;
-        } while ((r < stop) & (V != 0u));
-        if (last && r == nr) {
-          // the last cell: VE-FD the lesser of its edges, DFD its value; the decision its right
-          // edge's upper end (top edge on a transposed grid) if that edge is reached
-          const int cl = (C - 1) & 31;
-          double v;
-          if (KIND == K_DEC) {
-            const bool tr = sh->pd.tr != 0;
-            v = ((tr ? Y : V) >> cl) & 1u ? (tr ? at.t.y : at.r.y) : -2.0;
-          } else {
-            v = KIND == K_VEFD ? dmin(y, F) : y;
+      double y = dead, f = dead;
+      const int cl = (C - 1) & 31;  // the grid's last column in its block
+      const bool last = i == nbr - 1 && j == nbc - 1;
+      if (KIND == K_DEC || flat) {
+        int r = 0, by_row = 1;
+        while ((r < nr) & ((V | (r < 32 ? bmask >> r : 0u)) != 0u)) {
+          const int bad = walk_bits<KIND>(sh, slot, r, nr, bmask, bin, bout, F, V, omask, Y);
+          if (bad == nr) {
+            r = nr;
+            break;
           }
-          res = __shfl_sync(kFull, v, cl);
+          if constexpr (KIND == K_DEC) {
+            // the row that bits do not settle, with its values (the second time in a block 8
+            // rows, then the rest: such rows come together)
+            const int to = min(nr, bad + by_row);
+            by_row <<= 3;
+#pragma unroll 1
+            for (r = bad; r < to; ++r) {
+              walk_row(sh, slot, r, (bmask >> r) & 1u, bin[r], F, V, y, Y);
+              if ((lane == 31) & (int)(Y >> 31)) bout[r] = y;
+              omask |= (Y >> 31) << r;
+            }
+          }
+        }
+        if (r < nr) Y = 0u;
+      } else {
+        const int nc = min(32, C - (j << 5));
+        // (the row handed on goes to the list at once; without room, to the row not used)
+        double* out = on < kWalkCap ? sh->up_v[ob][on] : sh->spare_row;
+        walk_values<KIND>(sh, slot, nr, nc, upv, V, bmask, bin, bout, omask, out, y, f);
+        F = out[lane];
+        V = __ballot_sync(kFull, walk_live<KIND>(F));
+      }
+      if (last) {
+        // the last cell: VE-FD the lesser of its edges, DFD its value; the decision its right
+        // edge's upper end (top edge on a transposed grid) if that edge is reached
+        if (KIND == K_DEC) {
+          const bool tr = sh->pd.tr != 0;
+          const uint4 m = sh->mask[slot][nr - 1];
+          const int2 base = sh->base[slot][nr - 1];
+          const unsigned at = tr ? walk_place(base.y, m.y, cl) : walk_place(base.x, m.x, cl);
+          res = ((tr ? Y : V) >> cl) & 1u ? sh->vals[slot][at].y : -2.0;
+        } else if (flat) {
+          res = ((Y >> cl) & 1u) | (KIND == K_VEFD ? (V >> cl) & 1u : 0u) ? 0.0 : dead;
+        } else {
+          res = __shfl_sync(kFull, KIND == K_VEFD ? dmin(y, f) : y, nr - 1);
         }
       }
       if (status != WALK_OK) break;
@@ -896,6 +1068,7 @@ __device__ int walk_rows(const WaveArgs& wa, WalkShared* sh, Walk& w, int i0, in
     if (on == 0) break;
   }
   if (!walk_drop(wa, sh, w)) status = WALK_ERROR;
+  if (lane == 0) sh->cells += cells;
   __syncwarp();
   return status;
 }
@@ -958,11 +1131,12 @@ __device__ bool walk_start_row(const WaveArgs& wa, WalkShared* sh, Walk& w, int 
   const int lane = threadIdx.x & 31;
   const bool near = w.near_lo <= w.near_hi;
   if (lane == 0) {
+    sh->scan_to = 1;
     sh->scan_lo = near ? w.near_lo - 2 : 0;
     sh->scan_hi = near ? w.near_hi + 2 : INT_MAX - 1;
   }
   __syncwarp();
-  walk_request(sh, w, kScan, i, 1);
+  walk_request(sh, w, kScan, i);
   if (walk_take(wa, sh, w) < 0) return false;
   const int n = min(*(volatile int*)&sh->nup, kWalkCap);
   lost = near || *(volatile int*)&sh->lost != 0;
@@ -991,8 +1165,8 @@ __device__ void walk_cut(Walk& w, const WalkRecord* recs, int nbr, int nbc, int 
     if ((long long)mid + __ldcg(&recs[mid].hi) >= want) hi = mid;
     else lo = mid + 1;
   }
-  // (the band runs up and right, so these are in order; at least one row per piece)
-  lo = min(max(lo, q), nbr - pieces + q);
+  // (the band runs up and right, so these are in order; a long way along one row leaves pieces
+  // without rows)
   const int c0 = __shfl_sync(kFull, lo, 0), c1 = __shfl_sync(kFull, lo, 1);
   w.cut0 = m == 0 ? 0 : c0;
   w.cut1 = m + 1 >= pieces ? nbr : c1;
@@ -1051,6 +1225,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     sh->level = level;
     sh->rad = rad;
   }
+  sh->dead_row[lane] = dead;
   w.cur = 0;
   w.n = 0;
   w.blocks = 0;
@@ -1086,10 +1261,10 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     res = __ldcg(&q->res);
     return __ldcg(&q->gave_up) ? WALK_GIVE_UP : WALK_OK;
   }
-  const bool on = m < pieces;
-  WalkStat me{0.0, none, 1, 0, 0, 0, 0, 0};
+  const bool on = m < pieces && i0 < i1;
+  WalkStat me{0.0, none, on, 0, 0, 0, 0, !on};
   auto report = [&](int round) {
-    if (on && lane == 0) {
+    if (m < pieces && lane == 0) {
       WalkStat* q = g.stat[round & 1] + g.first + m;
       __stcg(&q->c, me.c);
       __stcg(&q->res, me.res);
@@ -1098,6 +1273,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
       __stcg(&q->empty, me.empty);
       __stcg(&q->part, me.part);
       __stcg(&q->gave_up, me.gave_up);
+      __stcg(&q->skip, me.skip);
     }
   };
   int first_empty = 0;
@@ -1132,10 +1308,12 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     if (!walk_barrier(wa, g)) return WALK_ERROR;
     // the round's reports
     const WalkStat* st = g.stat[round & 1] + g.first;
-    int moved = INT_MAX, bad = 0, hollow = INT_MAX, hollow_all = 0, part = 0;
+    int moved = INT_MAX, bad = 0, hollow = INT_MAX, hollow_all = 0, part = 0, end = 0;
     double cc = 0.0;
     for (int q = lane; q < pieces; q += 32) {
       const WalkStat* s = st + q;
+      if (__ldcg(&s->skip)) continue;
+      end = q;
       const int empty = __ldcg(&s->empty);
       bad |= __ldcg(&s->gave_up);
       if (round > 0 && __ldcg(&s->changed)) moved = min(moved, q);
@@ -1152,9 +1330,10 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
       bad |= __shfl_xor_sync(kFull, bad, d);
       hollow_all |= __shfl_xor_sync(kFull, hollow_all, d);
       part |= __shfl_xor_sync(kFull, part, d);
+      end = max(end, __shfl_xor_sync(kFull, end, d));
       cc = fmax(cc, __shfl_xor_sync(kFull, cc, d));
     }
-    const double last = __ldcg(&st[pieces - 1].res);
+    const double last = __ldcg(&st[end].res);
     int done = 0, rc = WALK_OK;
     if (bad) {
       done = 1;
@@ -1181,11 +1360,13 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
       rc = WALK_GIVE_UP;
     }
     int from = 0, again = 0;
+    int before = m - 1;  // the piece below this one
     if (!done && on && m > 0) {
-      again = round == 0 || __ldcg(&st[m - 1].changed);
-      from = __ldcg(&st[m - 1].which);
+      while (before > 0 && __ldcg(&st[before].skip)) --before;
+      again = round == 0 || __ldcg(&st[before].changed);
+      from = __ldcg(&st[before].which);
     }
-    if (done && rc == WALK_OK && res != none && on) {
+    if (done && rc == WALK_OK && res != none && m < pieces) {
       walk_cut(w, recs, nbr, nbc, pieces, m);
       o.band = true;
     }
@@ -1193,7 +1374,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     const int was = me.which;
     me.changed = 0;
     if (again) {
-      walk_load_end(sh, w, g.end[from] + g.first + m - 1);
+      walk_load_end(sh, w, g.end[from] + g.first + before);
       w.blocks = 0;
       c = 0.0;
       double r = none;

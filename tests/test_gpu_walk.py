@@ -26,6 +26,8 @@ def strips(built):
     (0, 2, 32, 33), (0, 3, 33, 32), (0, 2, 34, 65), (1, 3, 65, 64), (0, 2, 129, 128),
     (1, 2, 321, 40), (0, 3, 97, 700), (0, 2, 1025, 1023), (1, 3, 1500, 1400), (0, 2, 3000, 500),
     (1, 2, 1500, 40),   # a spacing far below the distance: a wide band
+    (1, 2, 2794, 44),   # ... along the block rows: long passes, pieces without rows
+    (0, 2, 44, 2794),
     (1, 3, 4100, 6007)])
 def test_walk_equals_strips_and_oracle(ctx, strips, built, style, d, n1, n2):
     P, Q = built.gen_pair(style, d, n1, n2, 100.0 if style else 1.0, 0.1, 91, n1)

@@ -1,7 +1,7 @@
 """CPU model of the walk sweeps' rules (rfd_walk.cuh), against the plain cell recurrences.
 
-Row rule: the decision's row of 32 columns by a carry chain of bits (walk_row) equals the
-recurrence cell by cell, on tie-heavy intervals.
+Block rule: the decision's rows of a block by carry chains of bits, as far as no value stands in
+the way of another (walk_bits), equal the recurrence cell by cell, on tie-heavy intervals.
 
 Group rule: pieces of a grid that start from everything that could be live (or from part of it),
 are walked again from their predecessor's end until a block row's list meets its record (up to
@@ -32,61 +32,90 @@ def serial_row(rl, ru, tl, tu, F, x):
     return out, x
 
 
-def bit_row(rl, ru, tl, tu, F, x):
-    """walk_row<K_DEC>: returns the same, and whether the column-by-column way was taken."""
-    n, full = 32, 0xffffffff
-    mr = sum(1 << j for j in range(n) if rl[j] >= 0.0)
-    mt = sum(1 << j for j in range(n) if tl[j] >= 0.0)
-    V = sum(1 << j for j in range(n) if F[j] < 2.0)
-    live_in = x < 2.0
-    prev = [x if j == 0 else tl[j - 1] for j in range(n)]
-    late = sum(1 << j for j in range(n) if tu[j] < prev[j])
-    gen = V & mt
-    X = ((mt + gen + int(live_in)) ^ mt ^ gen) & full
-    passing = X & ~V & mt & full
-    slow = bool(passing & (late | (passing << 1)))
-    y = [tl[j] if (V >> j) & 1 or not tl[j] < prev[j] else prev[j] for j in range(n)]
-    Y = mt & (V | X)
-    if slow:
-        y = [tl[j] if (mt >> j) & 1 and (V >> j) & 1 else DEAD for j in range(n)]
+def bit_block(rl, ru, tl, tu, F, xin):
+    """walk_bits<K_DEC> on rows 0 .. nr - 1: the rows settled by bits, what they hand on up (values)
+    and to the right (one value a row)."""
+    n, full, nr = 32, 0xffffffff, len(rl)
+
+    def bits(a):
+        return sum(1 << j for j in range(n) if a[j])
+    V = bits(F < 2.0)
+    above = bits((F < 2.0) & (F > 0.0))
+    rows = []
+    for r in range(nr):
+        mr, mt = bits(rl[r] >= 0.0), bits(tl[r] >= 0.0)
+        gen = V & mt
+        X = ((mt + gen + int(xin[r] < 2.0)) ^ mt ^ gen) & full
+        ok = mr & (X | V)
+        held = above & ~X
+        ends = bits((rl[r] >= 0.0) & (ru[r] < 1.0))
+        rows.append((X, ok, X & ~V & mt, mt & (X | V), ok & held & ends))
+        above = ok & (bits((rl[r] >= 0.0) & (rl[r] > 0.0)) | held)
+        V = ok
+
+    def run(c, r):
+        """Largest start from row r down to where column c's run began."""
+        f = 0.0
         while True:
-            xs = [x if live_in else DEAD] + y[:-1]
-            yn = []
-            for j in range(n):
-                up = (V >> j) & 1
-                ends = not (mt >> j) & 1 or (not up and tu[j] < xs[j])
-                yn.append(DEAD if ends else tl[j] if up or not tl[j] < xs[j] else xs[j])
-            moved = yn != y
-            y = yn
-            if not moved:
-                break
-        X = sum(1 << j for j in range(n) if xs[j] < 2.0)
-        Y = sum(1 << j for j in range(n) if y[j] < 2.0)
-    out = np.full(n, DEAD)
-    for j in range(n):
-        xl = (X >> j) & 1
-        if (mr >> j) & 1 and (xl or not ru[j] < F[j]):
-            out[j] = rl[j] if xl or not rl[j] < F[j] else F[j]
-    return out, (y[31] if Y >> 31 else DEAD), slow
+            if r < 0:
+                return max(f, F[c])
+            f = max(f, rl[r][c])
+            if rows[r][0] >> c & 1:
+                return f
+            r -= 1
+    out, nok = [], nr
+    for r, (X, ok, passing, Y, risk) in enumerate(rows):
+        ends = bits((tl[r] >= 0.0) & (tu[r] < 1.0)) | 1 << 31
+        x, before, clash = DEAD, -2, False
+        if passing & ends:
+            for c in range(n):
+                if passing >> c & 1:
+                    frm = x if before == c - 1 else xin[r] if c == 0 else tl[r][c - 1]
+                    clash |= tu[r][c] < frm
+                    x, before = max(tl[r][c], frm), c
+        for c in range(n):
+            if risk >> c & 1:
+                clash |= ru[r][c] < run(c, r - 1)
+        if clash:
+            nok = r
+            break
+        out.append((x if before == 31 else tl[r][31]) if Y >> 31 & 1 else DEAD)
+    up = F if nok == 0 else np.array(
+        [run(c, nok - 1) if rows[nok - 1][1] >> c & 1 else DEAD for c in range(n)])
+    return nok, up, out
 
 
-@pytest.mark.parametrize("levels,empty", [(3, 0.1), (3, 0.5), (8, 0.2), (1000, 0.05), (1000, 0.4)])
-def test_row_of_bits_equals_recurrence(levels, empty):
+@pytest.mark.parametrize("levels,empty,cut", [(3, 0.1, 0.1), (3, 0.5, 0.4), (8, 0.2, 0.02),
+                                              (1000, 0.05, 0.01), (1000, 0.4, 0.3)])
+def test_block_of_bits_equals_recurrence(levels, empty, cut):
     g = np.random.default_rng(levels + int(100 * empty))
-    slow = 0
-    for _ in range(1500):
+    whole = clashed = 0
+    for _ in range(300):
+        nr = int(g.integers(1, 33))
+
         def interval():
-            a = np.sort(g.integers(0, levels + 1, (2, 32)) / levels, axis=0)
-            gone = g.random(32) < empty
-            return np.where(gone, -1.0, a[0]), np.where(gone, -2.0, a[1])
+            a = np.sort(g.integers(0, levels + 1, (2, nr, 32)) / levels, axis=0)
+            gone, open_ = g.random((nr, 32)) < empty, g.random((2, nr, 32)) >= cut
+            lo, hi = np.where(open_[0], 0.0, a[0]), np.where(open_[1], 1.0, a[1])
+            return np.where(gone, -1.0, lo), np.where(gone, -2.0, hi)
         (rl, ru), (tl, tu) = interval(), interval()
         F = np.where(g.random(32) < g.random(), g.integers(0, levels + 1, 32) / levels, DEAD)
-        x = g.integers(0, levels + 1) / levels if g.random() < 0.5 else DEAD
-        want, xw = serial_row(rl, ru, tl, tu, F, x)
-        got, xg, s = bit_row(rl, ru, tl, tu, F, x)
-        slow += s
-        assert np.array_equal(want, got) and xw == xg
-    assert 0 < slow < 1500
+        xin = np.where(g.random(nr) < g.random(), g.integers(0, levels + 1, nr) / levels, DEAD)
+        r = 0
+        while r < nr:
+            n, up, out = bit_block(rl[r:], ru[r:], tl[r:], tu[r:], F, xin[r:])
+            whole += r == 0 and n == nr
+            for k in range(n):
+                F, x = serial_row(rl[r + k], ru[r + k], tl[r + k], tu[r + k], F, xin[r + k])
+                assert x == out[k]
+            assert np.array_equal(F, up)
+            r += n
+            if r < nr:  # a row with its values
+                G, x = serial_row(rl[r], ru[r], tl[r], tu[r], F, xin[r])
+                F = G
+                clashed += 1
+                r += 1
+    assert whole > 0 and clashed > 0
 
 
 # ------------------------------------------------------------------ group rule
