@@ -159,6 +159,7 @@ struct WaveArgs {
   int window_teams;  // ... and at least this over the active pairs (a lone pair: its teams)
   int kary_k;        // continuous search: radii per k-ary round (< 2: none)
   int kary_gate;     // ... run while at most this many pairs are active
+  int kary_tree;     // rounds of the next probes of a plain search instead (tree_arm)
 };
 
 // ------------------------------------------------------------------ memory helpers

@@ -358,23 +358,23 @@ __global__ void dfd_fill_kernel(const PairDesc* pairs, int npairs, int rows_per_
 // Marks the boundary rows of the 32-row strips of every pair about to run `phase` as not
 // yet written (VE-FD and decision launches; see kBndEmpty).  Grid as dfd_fill_kernel.
 // A gated probe round (WaveArgs.gate): the first block to look decides for the whole launch
-// whether enough pairs are still active (or a single one, which gains nothing from the
-// queue); true to run.  A skipped round does no work, so the rounds after it skip too.
-__device__ bool gate_open(int* gate, const int* active, int gate_min) {
+// whether enough pairs are still active (or, with lone, a single one, which gains nothing from
+// the queue unless it has tree rounds); true to run.  A skipped round does no work, so the rounds after it skip too.
+__device__ bool gate_open(int* gate, const int* active, int gate_min, int lone) {
   int d = ld_volatile(gate);
   if (d == 0) {
     const int a = ld_volatile(active);
-    atomicCAS(gate, 0, (a >= gate_min || a == 1) ? 1 : 2);
+    atomicCAS(gate, 0, (a >= gate_min || (a == 1 && lone)) ? 1 : 2);
     d = ld_volatile(gate);
   }
   return d == 1;
 }
 
 __global__ void bnd_fill_kernel(const PairDesc* pairs, const PairState* st, int npairs, int phase,
-                                int* gate, const int* active, int gate_min) {
+                                int* gate, const int* active, int gate_min, int lone) {
   if (gate) {
     __shared__ int open;
-    if (threadIdx.x == 0) open = gate_open(gate, active, gate_min);
+    if (threadIdx.x == 0) open = gate_open(gate, active, gate_min, lone);
     __syncthreads();
     if (!open) return;
   }
@@ -519,12 +519,87 @@ __device__ PairState* kary_member(const WaveArgs& wa, PairState* g, int m) {
   return m == 0 ? g : wa.st + g->kary_base + (m - 1);
 }
 
+// Rounds of the next probes (WaveArgs::kary_tree): the strips of a pair with one long and one
+// short curve are few, so its probe, a chain of the long curve's chunks (50,000 x 1,039 points:
+// 33 strips, 5.0 ms a probe), leaves most teams idle.  A round then decides the next two or three
+// probes of the search at once, for either outcome: node k's radius is what the search would
+// propose after the outcomes that lead there (2k + 1: unreachable, 2k + 2: reachable).  kary_done
+// takes the path that the outcomes give and leaves the other nodes out, so the radii, the
+// outcomes, the probe count and the nominal cells are the one-by-one search's.  Measured: that
+// pair's search 181 ms one by one, 70 ms with rounds of seven; the last pairs of 1,024 uneven
+// ones (up to 50,000 points) 142 ms against 83.
+// Node k of g's tree: the search before the node's probe, and its radius; false: not reached.
+__device__ bool tree_node(const PairState* g, int k, Search& q, double& eps) {
+  q = g->srch;
+  int depth = 0;
+  for (int v = k; v > 0; v = (v - 1) >> 1) ++depth;
+  for (int d = depth;; --d) {
+    if (!search_next(q, &eps)) return false;
+    if (d == 0) return true;
+    // the node's ancestor d - 1 levels up is a right child (even): the probe was reachable
+    const int v = ((k + 1) >> (d - 1)) - 1;
+    search_update(q, eps, (v & 1) == 0);
+  }
+}
+
+// The nodes of a tree round: as many as the teams have room for at once (a quarter of the strips
+// may wait), since past that two rounds of one probe cost the same and do less.
+__device__ int tree_arm(const WaveArgs& wa, PairState* g, int S) {
+  const long long load = (long long)S * max(1, ld_volatile(wa.active_pairs));
+  const long long teams = wa.window_teams + (wa.window_teams >> 2);
+  const int n = load * 7 <= teams ? 7 : load * 3 <= teams ? 3 : 1;
+  if (n == 1) return 1;
+  Search q;
+  double eps;
+  int m = 0;
+  for (int k = 1; k < n; ++k) {
+    PairState* ms = kary_member(wa, g, k);
+    ms->kary_in = 0;
+    if (!tree_node(g, k, q, eps)) continue;
+    ++m;
+    ms->split = eps;
+    ms->r2 = __dmul_rn(eps, eps);
+    ms->kary_in = 1;
+    ms->phase = PH_SEARCH;
+    ms->active = 1;
+  }
+  if (m == 0) return 1;
+  g->kary_in = 1;  // (its radius is set)
+  g->kary_n = n;
+  g->kary_left = m + 1;
+  __threadfence();
+  return n;
+}
+
+// Applies the outcomes of g's tree round along the search's path.
+__device__ void tree_done(const WaveArgs& wa, PairState* g) {
+  const int n = g->kary_n;
+  for (int k = 0; k < n;) {
+    double eps;
+    if (!search_next(g->srch, &eps)) break;
+    PairState* m = kary_member(wa, g, k);
+    const bool reach = ld_volatile(&m->kary_reach) != 0;
+    if (k > 0) {
+      g->cells_eval += m->cells_eval;
+      g->cells_fp64 += m->cells_fp64;
+      g->cells_nominal += m->cells_nominal;
+    }
+    search_update(g->srch, eps, reach);
+    k = 2 * k + 1 + reach;
+  }
+  for (int k = 1; k < n; ++k) {
+    PairState* m = kary_member(wa, g, k);
+    m->cells_eval = m->cells_fp64 = m->cells_nominal = 0;
+  }
+}
+
 // Sets up pair g's next probe (phase PH_SEARCH, split set by next_probe): a k-ary round's
 // members get their radii and states; returns the decisions of the round (1: one decision at
 // the split).  Queues nothing: a launch round takes the members' strips from its item list,
 // the continuous search queues them (start_next).  One thread.
-__device__ int kary_arm(const WaveArgs& wa, PairState* g) {
+__device__ int kary_arm(const WaveArgs& wa, PairState* g, int S) {
   int n = 1;
+  if (wa.kary_tree) return g->kary_cap > 0 ? tree_arm(wa, g, S) : 1;
   if (g->kary_cap > 0 && wa.kary_k >= 2 && g->srch.mode == SM_BISECT &&
       ld_volatile(wa.active_pairs) <= wa.kary_gate) {
     // the widest round whose decisions still close the gap within the probe cap: halvings
@@ -569,13 +644,14 @@ __device__ void start_armed(const WaveArgs& wa, PairState* g, int p, int S) {
     start_probe(wa, g, p, S);
     return;
   }
-  for (int k = 0; k < g->kary_n; ++k)
-    start_probe(wa, kary_member(wa, g, k), k == 0 ? p : g->kary_base + (k - 1), S);
+  const int n = g->kary_n;
+  for (int k = 0; k < n; ++k)
+    if (k == 0 || kary_member(wa, g, k)->kary_in) start_probe(wa, kary_member(wa, g, k), k == 0 ? p : g->kary_base + (k - 1), S);
 }
 
 // Continuous search: arms and starts pair p's next probe.  One thread.
 __device__ void start_next(const WaveArgs& wa, PairState* g, int p, int S) {
-  kary_arm(wa, g);
+  kary_arm(wa, g, S);
   start_armed(wa, g, p, S);
 }
 
@@ -588,31 +664,35 @@ __device__ void kary_done(const WaveArgs& wa, PairState* ms, int S, bool queue) 
   __threadfence();
   if (atomicSub(&g->kary_left, 1) != 1) return;
   __threadfence();
-  const int n = g->kary_n;
-  double ub = g->srch.ub, lb = g->srch.lb;
-  for (int k = 0; k < n; ++k) {
-    const PairState* m = kary_member(wa, g, k);
-    if (ld_volatile(&m->kary_reach) && m->split < ub) ub = m->split;
+  if (wa.kary_tree) {
+    tree_done(wa, g);
+  } else {
+    const int n = g->kary_n;
+    double ub = g->srch.ub, lb = g->srch.lb;
+    for (int k = 0; k < n; ++k) {
+      const PairState* m = kary_member(wa, g, k);
+      if (ld_volatile(&m->kary_reach) && m->split < ub) ub = m->split;
+    }
+    for (int k = 0; k < n; ++k) {
+      const PairState* m = kary_member(wa, g, k);
+      if (!ld_volatile(&m->kary_reach) && m->split < ub && m->split > lb) lb = m->split;
+    }
+    for (int k = 1; k < n; ++k) {
+      PairState* m = kary_member(wa, g, k);
+      g->cells_eval += m->cells_eval;
+      g->cells_fp64 += m->cells_fp64;
+      g->cells_nominal += m->cells_nominal;
+      m->cells_eval = m->cells_fp64 = m->cells_nominal = 0;
+    }
+    g->srch.lb = lb;
+    g->srch.ub = ub;
+    g->srch.probes += n;
   }
-  for (int k = 0; k < n; ++k) {
-    const PairState* m = kary_member(wa, g, k);
-    if (!ld_volatile(&m->kary_reach) && m->split < ub && m->split > lb) lb = m->split;
-  }
-  for (int k = 1; k < n; ++k) {
-    PairState* m = kary_member(wa, g, k);
-    g->cells_eval += m->cells_eval;
-    g->cells_fp64 += m->cells_fp64;
-    g->cells_nominal += m->cells_nominal;
-    m->cells_eval = m->cells_fp64 = m->cells_nominal = 0;
-  }
-  g->srch.lb = lb;
-  g->srch.ub = ub;
-  g->srch.probes += n;
   g->kary_n = 0;
   next_probe(g, wa.active_pairs);
   if (g->phase == PH_SEARCH && g->active) {
     if (queue) start_next(wa, g, p, S);
-    else kary_arm(wa, g);
+    else kary_arm(wa, g, S);
   }
 }
 
@@ -621,7 +701,9 @@ __global__ void search_queue_init_kernel(const PairDesc* pairs, PairState* st, i
                                          WaveArgs wa) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npairs; p += gridDim.x * blockDim.x) {
     if (st[p].phase != PH_SEARCH || !st[p].active) continue;
-    start_armed(wa, st + p, p, (pairs[p].n1 - 1 + 31) >> 5);
+    const int S = (pairs[p].n1 - 1 + 31) >> 5;
+    if (wa.kary_tree && st[p].kary_cap > 0) kary_arm(wa, st + p, S);
+    start_armed(wa, st + p, p, S);
   }
 }
 
@@ -732,8 +814,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) team_kernel(WaveArgs
           // launch rounds: the next launch runs what is armed here (its fill resets the rows)
           else if (KIND == K_DEC && !dyn && st->phase == PH_KWAIT) kary_done(wa, st, S, false);
           else if (KIND == K_DEC && !dyn && st->phase == PH_SEARCH && st->active &&
-                   st->kary_cap > 0)
-            kary_arm(wa, st);
+                   st->kary_cap > 0 && !wa.kary_tree)
+            kary_arm(wa, st, S);
         }
       }
     }
@@ -1675,21 +1757,47 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   int64_t nwin = twin ? (maxSt + twin - 1) / twin : 0;  // (recomputed for split pairs below)
   // Continuous search: a queue slot for every strip of every probe
   // (at most 512 MB; past that, and for the solo strips, one launch per probe round)
+  constexpr int64_t kSplitPairs = 8;
   int64_t dyn_cap = 0;
   if (mode == MODE_DISTANCE && max_probes > 1 && !ctx->solo && !ctx->lockstep && !twin) {
     for (int64_t p = 0; p < npairs; ++p)
       dyn_cap += (std::max<int64_t>(trows(p) - 1, 0) + 31) / 32 * max_probes;
     if (dyn_cap * (int64_t)sizeof(unsigned long long) > ((int64_t)512 << 20)) dyn_cap = 0;
   }
-  const size_t dyn_off = dyn_cap ? take(sizeof(unsigned long long) * dyn_cap) : 0;
   // k-ary rounds (rfd_options.search_arity = K): the pairs whose probe chains are longest get
   // K - 1 member decisions each (descriptor, state and boundary rows of their own, after the
   // pairs' in the same arrays).  A decision's chain is about max(strips x 7 us, 32-column
   // chunks x 3 us) on a B200.  The members of all pairs together use at most a quarter of
   // the device memory that is free or already the context's; a pair whose members would
   // exceed what is left gets none.
-  const int karity = (mode == MODE_DISTANCE && max_probes > 1 && !ctx->solo && !twin &&
-                      o.search_arity >= 2) ? std::min<int>(o.search_arity, RFD_MAX_ARITY) : 0;
+  const bool kuser = mode == MODE_DISTANCE && max_probes > 1 && !ctx->solo && !twin && o.search_arity >= 2;
+  // A pair with one long curve, kWalkAspect times the other's length, stays on the strips: rows along
+  // the shorter curve make them few, and a spacing far below the distance a band that is wide
+  // along the denser curve.
+  constexpr int kWalkAspect = 8, kWalkAspectFrom = 8192;
+  // Without search_arity, tree rounds (tree_arm): for the pairs that stay on the strips as long and thin
+  // ones, where two probes' worth of other strips fit beside a pair's own.
+  const bool walks = ctx->walk && !o.dense && !ctx->solo && !ctx->prof;
+  auto thin = [&](int64_t p) {
+    const int64_t hi = std::max(n1s[p], n2s[p]), lo = std::min(n1s[p], n2s[p]);
+    return walks && hi >= kWalkAspectFrom && hi >= kWalkAspect * lo;
+  };
+  auto tree_fits = [&](int64_t p) {
+    return thin(p) && n1s[p] >= 2 && n2s[p] >= 2 && (trows(p) - 1 + 31) / 32 * 3 <= ctx->team_grid[K_DEC] * 5 / 4;
+  };
+  bool ktree = walks && mode == MODE_DISTANCE && max_probes > 1 && dyn_cap && !kuser;
+  if (ktree) {
+    bool any = false;
+    for (int64_t p = 0; p < npairs; ++p) {
+      any = any || tree_fits(p);
+      // (a call that splits a pair, below, keeps to that)
+      if (npairs <= kSplitPairs && ctx->split_min > 0 &&
+          (trows(p) - 1 + 31) / 32 >= std::max(2, ctx->split_min))
+        ktree = false;
+    }
+    ktree = ktree && any;
+  }
+  int karity = kuser ? std::min<int>(o.search_arity, RFD_MAX_ARITY) : ktree ? 7 : 0;
   std::vector<int64_t> kpairs;
   if (karity) {
     size_t free_b = 0, total_b = 0;
@@ -1698,10 +1806,12 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       free_b = 0;
     }
     double room = 0.25 * ((double)free_b + (double)ctx->dws_size);
+    if (ktree) room = std::min(room, (double)(1ull << 30));
     std::vector<double> mbytes(npairs, 0.0);
     std::vector<std::pair<double, int64_t>> est;
     for (int64_t p = 0; p < npairs; ++p) {
       if (n1s[p] < 2 || n2s[p] < 2) continue;
+      if (ktree && !tree_fits(p)) continue;
       const int64_t St = (trows(p) - 1 + 31) / 32, C = tcols(p);
       const double bytes = 8.0 * (double)std::max<int64_t>(St - 1, 1) * (double)align_up((size_t)C, 32) +
                            4.0 * (double)std::max<int64_t>(St - 1, 1) * (double)(C / 32 + 64) +
@@ -1719,6 +1829,14 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       kpairs.push_back(est[k].second);
     }
   }
+  if (ktree && kpairs.empty()) {
+    ktree = false;
+    karity = 0;
+  }
+  // (a tree round of n nodes advances log2(n + 1) probes; the last one may advance fewer)
+  if (ktree)
+    for (int64_t p : kpairs) dyn_cap += (trows(p) - 1 + 31) / 32 * (4 * (int64_t)max_probes / 3 + 8);
+  const size_t dyn_off = dyn_cap ? take(sizeof(unsigned long long) * dyn_cap) : 0;
   const int64_t nmem = (int64_t)kpairs.size() * (karity > 1 ? karity - 1 : 0);
   // Meet in the middle (split_meet_kernel): in a call of at most kSplitPairs pairs, the chain
   // of a pair's team strips, which bounds a long pair's VE-FD and decisions, runs as two halves
@@ -1728,7 +1846,6 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   // k .. S - 1, which its forward half does not use, hold its mirror's rows (S rows in all,
   // one more than unsplit); the probe rounds run as launches.  Larger calls keep every team
   // busy with pairs already and keep the continuous search.
-  constexpr int64_t kSplitPairs = 8;
   std::vector<int64_t> ksp(npairs, 0);  // forward strips of a split pair (0: not split)
   std::vector<int64_t> mirror_of(npairs, -1);  // its mirror's descriptor index
   int64_t nsplit = 0, nfwd = 0, nmir = 0;  // split pairs; forward and mirror team items
@@ -1772,7 +1889,6 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   L.titems = take(sizeof(int2) * ntitems);
   // walk: pairs longest first, plans (host-made for the first launches, device-made for the
   // search's tail), the groups' words
-  const bool walks = ctx->walk && !o.dense && !ctx->solo && !ctx->prof;
   const size_t order_off = take(sizeof(int) * npairs);
   const size_t plan_off = take(sizeof(int) * (2 + npairs) * 3);
   const int64_t wg = walks ? ctx->walk_grid : 0;
@@ -1862,10 +1978,6 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   // walk groups: chunk bounds of the shorter curve and a record per block row of the longer one
   // (about 34 bytes a point), longest pairs first, within kWalkBytes in all; a pair without
   // them is walked by one CTA
-  // A pair with one long curve, kWalkAspect times the other's length, stays on the strips: rows along
-  // the shorter curve make them few, and a spacing far below the distance a band that is wide
-  // along the denser curve.
-  constexpr int kWalkAspect = 8, kWalkAspectFrom = 8192;
   constexpr size_t kWalkBytes = (size_t)1 << 30;
   std::vector<size_t> wball(npairs, 0), wrec(npairs, 0);
   std::vector<int> worder(npairs);
@@ -2017,8 +2129,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     s.blo = s.bhi = NAN;
     s.coarse = (ck && n1 >= 2 && n2 >= 2) ? 1 : 0;
     s.formula = formula[p];
-    s.walk_off = walks && std::max(n1, n2) >= kWalkAspectFrom &&
-                 std::max(n1, n2) >= kWalkAspect * std::min(n1, n2);
+    s.walk_off = thin(p);
     if (o.bracket && mode == MODE_DISTANCE) {
       s.blo = o.bracket[2 * p];
       s.bhi = o.bracket[2 * p + 1];
@@ -2366,7 +2477,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     const int fill_gx = std::max(32, 8 * ctx->num_sms / fill_gy);
     auto fill = [&](int ph) {
       bnd_fill_kernel<<<dim3(fill_gx, fill_gy), 256, 0, st>>>(dt, ds, (int)nst, ph, wa.gate,
-                                                               wa.active_pairs, wa.gate_min);
+                                                               wa.active_pairs, wa.gate_min, !ktree);
       ++launches;
     };
     // One VE-FD phase or probe round of the team strips: the rows reset and one launch, or
@@ -2514,6 +2625,8 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     if (ctx->timing) RFD_CUDA(record(2));
     const int nprobe = mode == MODE_DECIDE ? 1 : max_probes;
     wa.kary_k = karity;
+    wa.kary_tree = ktree;
+    wa.window_teams = ctx->team_grid[K_DEC];
     wa.kary_gate = kary_gate;
     if (dyn_cap) {
       // Probe rounds as single launches while many pairs are active (the rounds then keep
@@ -2538,7 +2651,6 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       wa.dyn_tail = counters + (L.nlaunch - 1);
       wa.dyn_cap = dyn_cap;
       wa.window = ctx->search_window;
-      wa.window_teams = ctx->team_grid[K_DEC];
       const int nstatic = wa.nitems;
       wa.nitems = 0;  // every strip comes from the queue
       fill(PH_SEARCH);
@@ -2591,7 +2703,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       return rc ? rc : read_back();
     }
     nwalk = 0;
-    const int search = nmem == 0 ? 4 : 0;
+    const int search = kuser && nmem ? 0 : 4;
     // The DFD stays on the strips with the coarse bound, whose level opens most of the coarse
     // grid, and where the pairs outnumber the CTAs: the strips then run at the FP64 rate
     // (5e11 cells/s), and the walk's few sweeps take as long; and where a pair has one curve
@@ -2644,7 +2756,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
                          ctx->solo, ctx->dfd_rows, ctx->dfd_skew, ctx->lockstep,
                          ctx->search_switch, ctx->search_window, ctx->team_warps,
                          (int)(ctx->spin_cycles >> 32),
-                         (int)(ctx->spin_cycles & 0xffffffff), karity, kary_gate, (int)twin,
+                         (int)(ctx->spin_cycles & 0xffffffff), karity, (int)ktree, kary_gate, (int)twin,
                          (int)nsplit, ctx->split_min, (int)walks};
     const void* ptrs[] = {dbase, hbase, gmodel, gmodel ? rfd_mlp::buffers_id(gmodel) : nullptr,
                           (const void*)st};
@@ -3620,7 +3732,7 @@ extern "C" int32_t rfd_decide_noalloc(const double* c1, int64_t n1, const double
   ka.quota = 1;
   walk_kernel<<<1, kWalkThreads, kWalkSmem, st>>>(wa, ka);
   RFD_CUDA(cudaGetLastError());
-  bnd_fill_kernel<<<dim3(256, 1), 256, 0, st>>>(ddesc, dstate, 1, PH_SEARCH, nullptr, nullptr, 0);
+  bnd_fill_kernel<<<dim3(256, 1), 256, 0, st>>>(ddesc, dstate, 1, PH_SEARCH, nullptr, nullptr, 0, 0);
   RFD_CUDA(cudaGetLastError());
   team_kernel<K_DEC, 8><<<nd.team_grid, kTeamThreads, team_smem_bytes<K_DEC>(), st>>>(wa);
   RFD_CUDA(cudaGetLastError());
