@@ -284,4 +284,186 @@ __device__ int dfd_strip(const WaveArgs& wa, const PairDesc& pd, PairState* st, 
   return status;
 }
 
+// ---- fed strips: one row per lane, the cell weights computed by other warps
+//
+// With few strips the sweep is a chain of steps (columns, and strips times their lag of 64
+// columns), and the warp that forms both the weights and the minima takes 140 cycles a step, with
+// the coarse bound's square root (a branch in every step) 300 or more.  Here a team of three
+// warps runs a strip: two feeders fill tiles of 32 steps x 32 rows of weights, one the even and
+// one the odd steps, and the sweeping warp's step is a load, a shuffle and two compare-and-selects
+// deep.  One barrier of the team's 96 threads a tile, two tiles in turn.
+// Before and after, one pair: 50,000 x 30 points 11.3 and 2.4 ms (rows along the shorter curve; 48
+// ns a step), 50,000 x 1,039 11.9 and 3.2 ms, 8,000 x 9,000 4.8 and 2.0 ms, 61 x 52 81 and 30 us;
+// coarse by 6: 31,000 x 30,000 2.9 and 1.3 ms, 200,000 x 200,000 19.5 and 11.6 ms.
+constexpr int kFedTeams = 2;                    // teams of a block
+constexpr int kFedThreads = 96 * kFedTeams;
+constexpr int kFedRing = 64;                    // columns a feeder keeps: 32c - 31 .. 32c + 31
+
+struct FedShared {
+  double tile[2][32][32];                       // weight of row `lane` at step u
+  double ring[2][4 * kFedRing];
+  int item_pair, item_strip;
+  int stop[2];  // written before the barrier of an even / odd tile, read after it
+};
+
+__device__ __forceinline__ void fed_sync(int team) {
+  asm volatile("bar.sync %0, 96;" ::"r"(team + 1) : "memory");
+}
+
+// Feeder h of strip s: tile c is ready at the c-th barrier, and is overwritten after the next.
+template <int D, bool INFL>
+__device__ int fed_weights(const PairDesc& pd, const int s, FedShared* sh, int team, int h) {
+  constexpr int DS = D + (INFL ? 1 : 0);
+  const int lane = threadIdx.x & 31;
+  const int R = pd.n1, C = pd.n2;
+  double* ring = sh->ring[h];
+  double p[DS], q[DS];
+  const int row = min(s * 32 + lane, R - 1);
+#pragma unroll
+  for (int e = 0; e < DS; ++e) p[e] = __ldg(pd.P + (size_t)row * DS + e);
+  auto fetch = [&](int c) {
+    const int j = min((c << 5) + lane, C - 1);
+#pragma unroll
+    for (int e = 0; e < DS; ++e) q[e] = __ldg(pd.Q + (size_t)j * DS + e);
+  };
+  auto stage = [&](int c) {
+    const int slot = ((c << 5) + lane) & (kFedRing - 1);
+#pragma unroll
+    for (int e = 0; e < DS; ++e) ring[e * kFedRing + slot] = q[e];
+  };
+  fetch(0);
+  stage(0);
+  __syncwarp();
+  const int nsteps = C + 31;
+  for (int c = 0; (c << 5) < nsteps; ++c) {
+    fetch(c + 1);
+    double(*tile)[32] = sh->tile[c & 1];
+#pragma unroll 4
+    for (int u = h; u < 32; u += 2) {
+      // (columns before the first: any weight, the sweep's step there is not used)
+      const int slot = max((c << 5) + u - lane, 0) & (kFedRing - 1);
+      double x[DS];
+#pragma unroll
+      for (int e = 0; e < DS; ++e) x[e] = ring[e * kFedRing + slot];
+      tile[u][lane] = cell_weight<D, INFL>(p, x);
+    }
+    __syncwarp();
+    stage(c + 1);
+    __syncwarp();
+    fed_sync(team);
+    if (*(volatile int*)&sh->stop[c & 1]) return 1;
+  }
+  return 0;
+}
+
+// Sweeping warp of strip s: dfd_strip's protocol and values with K = 1, skewed.  A cell's value
+// handed up, min(max(w, min(left, b)), b), is formed as min(b, max(w, left)), which is the same
+// number and one operation less after `left`.
+__device__ inline int fed_strip(const WaveArgs& wa, const PairDesc& pd, PairState* st, const int s,
+                                FedShared* sh, int team) {
+  const int lane = threadIdx.x & 31;
+  const int R = pd.n1, C = pd.n2;
+  const int S = (R + 31) / 32;
+  const bool has_prod = s > 0, has_cons = s + 1 < S;
+  const int nring = pd.ring;
+  const int slot_in = has_prod ? (s - 1) % nring : 0;
+  const int slot_out = has_cons ? s % nring : 0;
+  int status = !ring_check(wa, slot_in >= 0 && slot_in < nring && slot_out >= 0 && slot_out < nring, 8);
+  double* in_bnd = has_prod ? pd.bnd + (size_t)slot_in * pd.cstride : nullptr;
+  double* out_bnd = has_cons ? pd.bnd + (size_t)slot_out * pd.cstride : nullptr;
+  unsigned long long* clr_in = has_prod ? pd.slots + (s - 1) : nullptr;
+  unsigned long long* clr_out = pd.slots + s;
+  unsigned long long* clr_next =
+      has_prod && s - 1 + nring < S ? pd.slots + (s - 1 + nring) : nullptr;
+  unsigned in_ok = 0, out_ok = 0;
+  constexpr int kPublish = 8;
+  Waiter wt;
+  wt.start(wa, st, s);
+  const int rlast = R - 1 - s * 32;
+  const bool holds_last = s == S - 1 && lane == rlast;
+  const int tres = C - 1 + lane;
+  double bot = kFltMax, carry = kFltMax, res = kFltMax;
+  const int nsteps = C + 31;
+  auto load_in = [&](int c) -> unsigned long long {
+    const int col = (c << 5) + lane;
+    if (!has_prod) return __double_as_longlong(col == 0 ? 0.0 : kFltMax);
+    if ((c << 5) >= C || col >= C) return __double_as_longlong(kFltMax);
+    if (in_ok < (unsigned)min((c + 1) << 5, C)) return kBndEmpty;
+    return ld_relaxed_u64(in_bnd + col);
+  };
+  auto cleared = [&](unsigned long long* cnt, unsigned have) -> unsigned {
+    const unsigned long long w = bcast(lane == 0 ? ld_acquire(cnt) : 0ull);
+    __syncwarp();
+    return max(have, (unsigned)w);
+  };
+  const bool store_out = has_cons && lane == 31;
+  auto steps = [&](const int c, const double inreg, auto first) {
+    constexpr bool FIRST = decltype(first)::value;
+    const double(*tile)[32] = sh->tile[c & 1];
+#pragma unroll 8
+    for (int u = 0; u < 32; ++u) {
+      const int t = (c << 5) + u;
+      const double w = tile[u][lane];
+      const double lin = __shfl_sync(kFull, inreg, u);
+      const double lup = __shfl_up_sync(kFull, carry, 1);
+      const double left = lane == 0 ? lin : lup;
+      const double b = FIRST && t == lane ? kFltMax : bot;
+      bot = dmax(w, dmin(left, b));
+      carry = dmin(dmax(w, left), b);
+      res = t == tres ? bot : res;
+      const int jo = t - 31;
+      if (store_out & ((unsigned)jo < (unsigned)C)) st_relaxed_f64(out_bnd + jo, carry);
+    }
+  };
+  unsigned long long nxt = load_in(0);
+  for (int c = 0; (c << 5) < nsteps; ++c) {
+    unsigned long long cur = nxt;
+    const bool reads = has_prod && (c << 5) < C;
+    const unsigned need_in = (unsigned)min((c + 1) << 5, C);
+    for (int it = 0; !status; ++it) {
+      if (reads && in_ok < need_in) {
+        in_ok = cleared(clr_in, in_ok);
+        if (in_ok >= need_in) cur = load_in(c);
+      }
+      if (__all_sync(kFull, cur != kBndEmpty)) break;
+      if (wt.check(it)) status = 1;
+      if (cur == kBndEmpty) cur = load_in(c);
+    }
+    if (reads && !status) {
+      const int col = (c << 5) + lane;
+      if (col < C) st_relaxed_u64(reinterpret_cast<unsigned long long*>(in_bnd) + col, kBndEmpty);
+      if ((c & (kPublish - 1)) == kPublish - 1 && clr_next) {
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence();
+          st_release(clr_next, need_in);
+        }
+      }
+    }
+    if (has_cons) {
+      const unsigned need_out = (unsigned)min(max((c << 5) + 1, 0), C);
+      for (int it = 0; !status && out_ok < need_out; ++it) {
+        out_ok = cleared(clr_out, out_ok);
+        if (out_ok >= need_out) break;
+        if (wt.check(it)) status = 1;
+      }
+    }
+    nxt = status ? 0ull : load_in(c + 1);  // in flight during this chunk
+    if (lane == 0) sh->stop[c & 1] = status;
+    fed_sync(team);  // tile c is ready; the feeders leave with this warp
+    if (status) return status;
+    if (c == 0) steps(c, __longlong_as_double(cur), BoolC<true>{});
+    else steps(c, __longlong_as_double(cur), BoolC<false>{});
+  }
+  if (clr_next) {
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      st_release(clr_next, kSlotAll);
+    }
+  }
+  if (holds_last) st->result = res;
+  return 0;
+}
+
 }  // namespace rfd

@@ -476,6 +476,58 @@ __global__ void __launch_bounds__(kBlock) dfd_kernel(WaveArgs wa) {
   }
 }
 
+// The same with 32-row strips run by teams of three warps (rfd_dfd.cuh, fed strips).
+template <bool INFL>
+__global__ void __launch_bounds__(kFedThreads) dfd_fed_kernel(WaveArgs wa) {
+  __shared__ FedShared shared[kFedTeams];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int team = warp / 3, role = warp % 3;
+  FedShared* sh = shared + team;
+  for (;;) {
+    if (role == 0) {
+      int pair = -1, strip = 0;
+      if (lane == 0) {
+        while (ld_volatile(wa.active_pairs) != 0 && !ld_volatile(wa.error)) {
+          const unsigned t = atomicAdd(wa.ticket, 1u);
+          if ((int)t >= wa.nitems) break;
+          const int2 it = wa.items[t];
+          const PairState* st = wa.st + it.x;
+          if (ld_volatile(&st->phase) != PH_DFD || !ld_volatile(&st->active)) continue;
+          if (it.y >= (wa.pairs[it.x].n1 + 31) / 32) continue;
+          pair = it.x;
+          strip = it.y;
+          break;
+        }
+        sh->item_pair = pair;
+        sh->item_strip = strip;
+      }
+    }
+    fed_sync(team);
+    const int p = sh->item_pair, s = sh->item_strip;
+    if (p < 0) return;
+    const PairDesc pd = wa.pairs[p];
+    PairState* st = wa.st + p;
+    if (role > 0) {
+      if (pd.d == 2 ? fed_weights<2, INFL>(pd, s, sh, team, role - 1)
+                    : fed_weights<3, INFL>(pd, s, sh, team, role - 1))
+        return;
+    } else {
+      if (fed_strip(wa, pd, st, s, sh, team)) return;
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence();
+        const int n = atomicAdd(&st->done_count, 1);
+        if (n == (pd.n1 + 31) / 32 - 1) {
+          __threadfence();
+          finalize<K_DFD>(st, pd, wa.active_pairs);
+          __threadfence();
+        }
+      }
+    }
+    fed_sync(team);  // the strip's item, stop word and tiles are free again
+  }
+}
+
 // Continuous search: waits (bounded) for queue slot k to be published and returns its pair
 // index; -1 when every pair is done, on an error, or when the wait runs out (which sets the
 // error word).
@@ -1399,6 +1451,7 @@ struct rfd_context {
   int dfd_skew = -1;   // RFD_DFD_SKEW: 1 skewed rows, 0 stacked, unset: chosen per call
   int dfd_grid[2] = {0, 0};  // [stacked, skewed] for dfd_rows
   int dfd_grid_all[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};  // for rows 1, 2, 4, 8
+  int fed_grid[2] = {0, 0};  // fed strips: plain, inflated
   int dfd_grid_infl[2] = {0, 0};  // inflated coarse sweep, 1 row per lane
   int prof = 0;  // RFD_PROF=1: team-strip cycle counters printed to stderr after each call
   // rows of the DFD strips' boundary ring per pair (RFD_DFD_RING_ROWS, at least 2; see
@@ -1929,7 +1982,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     const int64_t tstride = align_up((size_t)((tcols(p) + 31) / 32), 32);
     L.tags[p] = take(sizeof(unsigned) * L.ring_t[p] * tstride);
     L.prog[p] = take(sizeof(Prog) * std::max<int64_t>(St, (trows(p) + 31) / 32));
-    L.slots[p] = take(sizeof(unsigned long long) * (n1s[p] + 31) / 32);  // a count per DFD strip
+    L.slots[p] = take(sizeof(unsigned long long) * (std::max(n1s[p], trows(p)) + 31) / 32);  // a count per DFD strip
   }
   std::vector<size_t> mtags(nmem), mprog(nmem), mbnd(nmem);
   for (int64_t v = 0; v < nmem; ++v) {
@@ -2559,8 +2612,26 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       // the DFD sweep runs on the coarse pairs when the coarse upper bound is asked for
       const PairDesc* ddfd = ck ? (const PairDesc*)(dbase + cdescs) : dd;
       // The coarse pair has k times fewer points per curve: one row per lane gives its sweep
-      // the most strips in flight (long pair, k = 6: 21 ms against 38 with four rows).
-      const int rows = ck ? 1 : ctx->dfd_rows;
+      // the most strips in flight (long pair, k = 6, strips not fed: 21 ms against 38 with four
+      // rows).
+      // Fed strips (one row per lane) where all of them fit the chip at once: the sweep is then
+      // a chain of strips and columns, 2.4 to 4.6 times faster than with eight rows a lane (at
+      // more strips the sweep is bound by its instructions, and eight stacked rows take fewest);
+      // with the rows along the shorter curve, as the team strips', unless the pair is split or
+      // on the coarse grid.
+      bool turn = !ck && !nsplit && !twin;
+      // (a ring has two rows at least, or one for each row handed on: the team strips of 65 points
+      // hand on one, the DFD's two)
+      for (int64_t p = 0; p < npairs && turn; ++p)
+        turn = L.ring_t[p] >= std::min<int64_t>(2, (trows(p) + 31) / 32 - 1);
+      int64_t fstrips = 0;
+      for (int64_t p = 0; p < npairs; ++p) {
+        const int64_t r = ck && n1s[p] >= 2 && n2s[p] >= 2 ? coarse_n(n1s[p]) : turn ? trows(p) : n1s[p];
+        fstrips += (r + 31) / 32;
+      }
+      const bool fed = ctx->dfd_skew < 0 && fstrips <= (int64_t)ctx->fed_grid[ck > 0] * kFedTeams;
+      if (fed && turn) ddfd = dt;
+      const int rows = ck || fed ? 1 : ctx->dfd_rows;
       {
         const int gy = (int)std::min<int64_t>(npairs, 8 * ctx->num_sms);
         const int gx = std::max(32, 8 * ctx->num_sms / gy);
@@ -2568,9 +2639,13 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       }
       ++launches;
       wa.pairs = ddfd;  // the DFD sweep: given orientation, its own item list
-      wa.items = (const int2*)(dbase + L.items);
-      wa.nitems = L.nitems;
-      {
+      wa.items = (const int2*)(dbase + (fed && turn ? L.titems : L.items));
+      wa.nitems = fed && turn ? L.ntitems : L.nitems;
+      if (fed) {
+        const int g = (int)std::min<int64_t>(ctx->fed_grid[ck > 0], (fstrips + kFedTeams - 1) / kFedTeams);
+        if (ck) dfd_fed_kernel<true><<<g, kFedThreads, 0, st>>>(wa);
+        else dfd_fed_kernel<false><<<g, kFedThreads, 0, st>>>(wa);
+      } else {
         // skewed rows when the strips cannot fill the resident warps twice over (the sweep's
         // latency decides), stacked rows otherwise (instruction throughput decides)
         int64_t strips = 0;
@@ -3092,6 +3167,12 @@ int32_t rfd_context_create(int32_t device, rfd_context** out) {
       if (sk) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&od, dfd_kernel<1, true, true>, kBlock, 0);
       else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&od, dfd_kernel<1, false, true>, kBlock, 0);
       c->dfd_grid_infl[sk] = std::max(1, od) * c->num_sms;
+    }
+    for (int k = 0; k < 2; ++k) {
+      int od = 0;
+      if (k) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&od, dfd_fed_kernel<true>, kFedThreads, 0);
+      else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&od, dfd_fed_kernel<false>, kFedThreads, 0);
+      c->fed_grid[k] = std::max(1, od) * c->num_sms;
     }
     const char* pe = getenv("RFD_PROF");
     c->prof = pe && pe[0] == '1';
