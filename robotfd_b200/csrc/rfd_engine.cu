@@ -1448,6 +1448,7 @@ struct rfd_context {
   int search_switch = 0;  // active pairs below which the continuous search takes over
   int search_window = 2;  // continuous search: strips a probe queues ahead of its band
   int dfd_rows = 8;    // rows per lane of the DFD strips (RFD_DFD_ROWS = 1, 2, 4 or 8)
+  int dfd_auto = 1;    // neither set by RFD_DFD_ROWS nor tuned
   int dfd_skew = -1;   // RFD_DFD_SKEW: 1 skewed rows, 0 stacked, unset: chosen per call
   int dfd_grid[2] = {0, 0};  // [stacked, skewed] for dfd_rows
   int dfd_grid_all[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};  // for rows 1, 2, 4, 8
@@ -2631,7 +2632,16 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       }
       const bool fed = ctx->dfd_skew < 0 && fstrips <= (int64_t)ctx->fed_grid[ck > 0] * kFedTeams;
       if (fed && turn) ddfd = dt;
-      const int rows = ck || fed ? 1 : ctx->dfd_rows;
+      // Batches: four stacked rows a lane while the strips of eight are at most ten times the
+      // resident warps (the long pairs' strips, a chain, then end sooner: 1,024 uneven pairs
+      // 21.6 and 17.7 ms, 192 pairs 6.9 and 4.9, 256 short ones 0.98 and 0.52), eight past that
+      // (3,000 uneven pairs: 36.9 ms against 40.5).  Not with RFD_DFD_ROWS or a tuned shape.
+      int64_t strips8 = 0;
+      for (int64_t p = 0; p < npairs; ++p) strips8 += (n1s[p] + 255) / 256;
+      const bool four = !ck && !fed && ctx->dfd_auto && ctx->dfd_skew < 0 && npairs > kSplitPairs &&
+                        strips8 * 8 >= (int64_t)ctx->dfd_grid_all[2][0] * (kBlock / 32) &&
+                        strips8 <= (int64_t)ctx->dfd_grid_all[3][0] * (kBlock / 32) * 10;
+      const int rows = ck || fed ? 1 : four ? 4 : ctx->dfd_rows;
       {
         const int gy = (int)std::min<int64_t>(npairs, 8 * ctx->num_sms);
         const int gx = std::max(32, 8 * ctx->num_sms / gy);
@@ -2653,11 +2663,11 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
           const int64_t n1 = ck && n1s[p] >= 2 && n2s[p] >= 2 ? coarse_n(n1s[p]) : n1s[p];
           strips += (n1 + 32 * rows - 1) / (32 * rows);
         }
-        const int* grid = ck ? ctx->dfd_grid_infl : ctx->dfd_grid;
-        const int sk = ctx->dfd_skew >= 0 ? ctx->dfd_skew
+        const int* grid = ck ? ctx->dfd_grid_infl : four ? ctx->dfd_grid_all[2] : ctx->dfd_grid;
+        const int sk = four ? 0 : ctx->dfd_skew >= 0 ? ctx->dfd_skew
                                            : (strips < 2 * (int64_t)grid[1] * (kBlock / 32) ? 1 : 0);
         const int g = grid[sk];
-        switch (ck ? 100 + sk : ctx->dfd_rows * 2 + sk) {
+        switch (ck ? 100 + sk : rows * 2 + sk) {
           case 100: dfd_kernel<1, false, true><<<g, kBlock, 0, st>>>(wa); break;
           case 101: dfd_kernel<1, true, true><<<g, kBlock, 0, st>>>(wa); break;
           case 2: dfd_kernel<1, false><<<g, kBlock, 0, st>>>(wa); break;
@@ -3143,7 +3153,7 @@ int32_t rfd_context_create(int32_t device, rfd_context** out) {
     if (sn && atoi(sn) >= 1) c->search_window = atoi(sn);
     const char* dr = getenv("RFD_DFD_ROWS");
     if (dr && (dr[0] == '1' || dr[0] == '2' || dr[0] == '4' || dr[0] == '8') && !dr[1])
-      c->dfd_rows = dr[0] - '0';
+      c->dfd_rows = dr[0] - '0', c->dfd_auto = 0;
     const char* dk = getenv("RFD_DFD_SKEW");
     if (dk && (dk[0] == '0' || dk[0] == '1') && !dk[1]) c->dfd_skew = dk[0] - '0';
     for (int ri = 0; ri < 4; ++ri)

@@ -60,3 +60,17 @@ def test_fed_strips_of_several_pairs(both, built, coarse):
     a = [[r["dfd"] for r in c.distance_batch(Ps, Qs, **kw)] for c in both]
     assert a[0] == a[1] == a[2]
     assert a[0] == [r["dfd"] for r in both[0].distance_batch(Ps, Qs, **{**kw, "graph": True})]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("npairs,longest", [(9, 60000), (40, 9000), (500, 900)])
+def test_batches_on_either_side_of_the_rows_rule(built, both, npairs, longest):
+    """Four or eight rows a lane, by the strips of the call, against eight skewed."""
+    g = np.random.default_rng(npairs)
+    pairs = []
+    for k in range(npairs):
+        n1 = int(g.integers(longest // 2, longest))
+        pairs.append(built.gen_pair(k % 2, 2 + k % 2, n1, int(g.integers(2, 300)), 1.0, 0.1, 98, k))
+    Ps, Qs = [p for p, _ in pairs], [q for _, q in pairs]
+    a = [[r["dfd"] for r in c.distance_batch(Ps, Qs, precise=True, max_probes=1)] for c in both]
+    assert a[0] == a[1] == a[2]
