@@ -1590,7 +1590,8 @@ double pair_workspace_bytes(const rfd_context* ctx, int64_t n1, int64_t n2, int 
              + 8.0 * ring_words                           // boundary ring
              + 4.0 * rt * (double)(cols / 32 + 64)        // tags
              + 40.0 * (double)(St + 1) + 16.0 * (double)(n1 / 32 + rows / 32 + 2)  // progress, items
-             + 24.0 * (rt + rd) + 8192.0;                 // slot words, descriptors, state
+             + 24.0 * (rt + rd) + 8192.0                  // slot words, descriptors, state
+             + (ctx->walk ? 33.0 * (double)cols + (double)rows + 2048.0 : 0.0);  // walk records, bounds
   if (ck) b += 8.0 * (double)(d + 1) * (double)(n1 + n2) / ck + 16384.0;
   return b;
 }

@@ -38,8 +38,14 @@
 // piece that ends empty from everything that could be live ends the sweep (walk_sweep).  Once a
 // sweep has found the band, the next ones start their pieces only near where it ran.
 //
-// A sweep whose band is not thin (list overflow, block budget) gives up; the pair's phase then
-// runs on the strips as before.
+// A sweep whose band is not thin (list overflow, effort against progress) gives up; the pair's
+// phase then runs on the strips as before.
+//
+// What bounds it: the chain of a band's blocks.  A decision's block takes about 5,300 cycles (the
+// rows 2,900, waiting for the tile 900, the next block's choice 500; a tile is ready 3,500 after
+// its request), a VE-FD or DFD block with values about 10,000.  Against the strips, one pair:
+// search of 20,000 x 19,000 points 155 ms and 4.6 (37 probes), 2,000 x 1,900 17 and 2.7; bounds of
+// 60,000 x 45,000 points 35 and 1.8; VE-FD and one decision of 200,000 x 200,000 90 and 7.0.
 #pragma once
 
 #include "rfd_device.cuh"
