@@ -51,6 +51,7 @@
 #include "rfd_device.cuh"
 #include "rfd_filter.h"
 #include "rfd_team.cuh"
+#include "rfd_walk_cut.h"
 
 namespace rfd {
 
@@ -70,7 +71,6 @@ constexpr int kWalkVals = 2048;
 
 // A block row's output list as recorded by the first walk of a piece (n < 0: too long to record),
 // and the chunks lo .. hi of the list as last walked.
-constexpr int kWalkStretch = 10;
 constexpr int kWalkRec = 4;
 struct WalkRecord {
   int n, lo, hi, pad;
@@ -1157,25 +1157,18 @@ __device__ bool walk_start_row(const WaveArgs& wa, WalkShared* sh, Walk& w, int 
   return true;
 }
 
-// The piece of member m by where the band of an earlier sweep ran, from the records: block row i
-// ends about i + (its list's last chunk) blocks along it.  Pieces take equal stretches: piece q
-// starts with the first row that ends past q / pieces of the way (a bisection; the same for both
-// its neighbours, since no record changes meanwhile).
+// The piece of member m by where the band of an earlier sweep ran, from the records (walk_cut_row;
+// the same for both its neighbours, since no record changes meanwhile).
 __device__ void walk_cut(Walk& w, const WalkRecord* recs, int nbr, int nbc, int pieces, int m) {
   const int lane = threadIdx.x & 31;
   const int q = m + (lane & 1);  // lane 0: this piece's start, lane 1: its end
-  int lo = 0, hi = nbr;
-  const long long want = (long long)(nbr + nbc) * q / pieces;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if ((long long)mid + __ldcg(&recs[mid].hi) >= want) hi = mid;
-    else lo = mid + 1;
-  }
+  const int row = q > 0 && q < pieces
+                      ? walk_cut_row(q, pieces, nbr, nbc, [&](int i) { return __ldcg(&recs[i].hi); })
+                      : q > 0 ? nbr : 0;
   // (the band runs up and right, so these are in order; a long way along one row leaves pieces
   // without rows)
-  const int c0 = __shfl_sync(kFull, lo, 0), c1 = __shfl_sync(kFull, lo, 1);
-  w.cut0 = m == 0 ? 0 : c0;
-  w.cut1 = m + 1 >= pieces ? nbr : c1;
+  w.cut0 = __shfl_sync(kFull, row, 0);
+  w.cut1 = __shfl_sync(kFull, row, 1);
   w.near_lo = 0;
   w.near_hi = -1;
   if (w.cut0 > 0) {
@@ -1184,10 +1177,9 @@ __device__ void walk_cut(Walk& w, const WalkRecord* recs, int nbr, int nbc, int 
   }
 }
 
-// The number of pieces of a grid: of at least kWalkStretch blocks of a thin band (shorter ones
-// end before the band has forgotten their start).
+// (a pair without room for records is one piece)
 __device__ __forceinline__ int walk_pieces(const PairDesc& pd, int size, int nbr, int nbc) {
-  return pd.recs ? max(1, min(min(size, nbr / 2), (nbr + nbc) / kWalkStretch)) : 1;
+  return pd.recs ? walk_pieces(size, nbr, nbc) : 1;
 }
 
 // Options of a sweep.  flat: only whether a path survives the level (every live value 0): its

@@ -1,0 +1,39 @@
+"""Walk sweeps of a group of CTAs (rfd_walk.cuh) against the strips (RFD_WALK=0), where the pieces of
+the grid are cut in uncommon ways."""
+import numpy as np
+import pytest
+
+KEYS = ("distance", "dfd", "vefd", "endpoint", "lb", "ub", "probes", "flags", "cells_nominal")
+
+
+@pytest.fixture(scope="module")
+def strips(built):
+    import os
+    os.environ["RFD_WALK"] = "0"
+    try:
+        c = built.Context(0)
+    finally:
+        del os.environ["RFD_WALK"]
+    yield c
+    c.close()
+
+
+def check(ctx, strips, P, Q):
+    a, b = ctx.distance(P, Q, precise=True), strips.distance(P, Q, precise=True)
+    assert [a[k] for k in KEYS] == [b[k] for k in KEYS]
+    assert ctx.bounds(P, Q, quirks=False) == strips.bounds(P, Q, quirks=False)
+    for r in np.geomspace(0.5 * a["distance"], 1.2 * a["dfd"], 5):
+        assert ctx.decide(P, Q, r) == strips.decide(P, Q, r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [2, 3])
+@pytest.mark.parametrize("dwell,n,m", [(400, 2500, 1400), (1000, 4000, 2600), (700, 1500, 760)])
+def test_band_far_along_the_first_row(ctx, strips, built, d, dwell, n, m):
+    """A track that waits at its start: the band runs along the first block row past the first
+    piece's share of it."""
+    P, Q = built.gen_pair(0, d, n, m - dwell, 1.0, 0.05, 96, n)
+    g = np.random.default_rng(dwell)
+    Q = np.concatenate([Q[0] + 0.01 * g.standard_normal((dwell, d)), Q])
+    check(ctx, strips, P, Q)
+    check(ctx, strips, Q, P)
