@@ -928,6 +928,9 @@ __device__ __forceinline__ bool walk_skips_vefd(int quirks, const PairDesc& pd) 
 
 // The phases of one pair, one after another, as far as the walk takes them, by the CTAs of a
 // group together: every member comes to the same results, the first one keeps the pair's state.
+// It writes the state only after a barrier that the members pass once they have read it, and they
+// read it again only after the next one: every phase passes at least one barrier before its
+// finalize, and one after it.
 // Returns false on an error (the error word is set).
 __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh, Walk& w,
                           WalkGroup& g, int p) {
@@ -1037,6 +1040,9 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
       w.rounds = 0;
       for (;; rad *= 2.0) {
         if (ve > 0.0) {
+          // (no sweep, so no barrier yet: the first member's finalize must not run ahead of the
+          // others' reads of the phase)
+          if (!walk_barrier(wa, g)) return false;
           res = ve <= U ? ve : kFltMax;
           break;
         }
