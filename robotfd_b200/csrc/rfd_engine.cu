@@ -981,7 +981,7 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
     const int nbr = (sh->pd.n1 + 30) >> 5, nbc = (sh->pd.n2 + 30) >> 5;
     const int np = walk_pieces(sh->pd, g.size, nbr, nbc);
     if (np > 1 && g.rank < np)
-      walk_cut(w, (const WalkRecord*)sh->pd.recs, nbr, nbc, np, g.rank);
+      walk_cut(w, sh->pd, nbr, nbc, np, g.rank);
     if (!walk_barrier(wa, g)) return false;  // (before a record changes)
   }
   // a radius to grow a level from: the larger of the endpoint bound and f x the points' spacing

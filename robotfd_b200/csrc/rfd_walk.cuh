@@ -1159,12 +1159,14 @@ __device__ bool walk_start_row(const WaveArgs& wa, WalkShared* sh, Walk& w, int 
 
 // The piece of member m by where the band of an earlier sweep ran, from the records (walk_cut_row;
 // the same for both its neighbours, since no record changes meanwhile).
-__device__ void walk_cut(Walk& w, const WalkRecord* recs, int nbr, int nbc, int pieces, int m) {
+__device__ void walk_cut(Walk& w, const PairDesc& pd, int nbr, int nbc, int pieces, int m) {
   const int lane = threadIdx.x & 31;
+  const WalkRecord* recs = (const WalkRecord*)pd.recs;
   const int q = m + (lane & 1);  // lane 0: this piece's start, lane 1: its end
-  const int row = q > 0 && q < pieces
-                      ? walk_cut_row(q, pieces, nbr, nbc, [&](int i) { return __ldcg(&recs[i].hi); })
-                      : q > 0 ? nbr : 0;
+  const int row =
+      q > 0 && q < pieces
+          ? walk_cut_row(q, pieces, pd.n1, nbr, nbc, [&](int i) { return __ldcg(&recs[i].hi); })
+          : q > 0 ? nbr : 0;
   // (the band runs up and right, so these are in order; a long way along one row leaves pieces
   // without rows)
   w.cut0 = __shfl_sync(kFull, row, 0);
@@ -1365,7 +1367,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
       from = __ldcg(&st[before].which);
     }
     if (done && rc == WALK_OK && res != none && m < pieces) {
-      walk_cut(w, recs, nbr, nbc, pieces, m);
+      walk_cut(w, sh->pd, nbr, nbc, pieces, m);
       o.band = true;
     }
     if (done) return rc;
