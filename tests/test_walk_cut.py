@@ -35,8 +35,11 @@ def band(g, nbr, nbc):
     row."""
     hi = np.sort(g.integers(0, nbc, nbr))
     hi[g.integers(0, nbr + 1):] = nbc - 1     # along a row, then straight up
-    if g.random() < 0.3:
+    u = g.random()
+    if u < 0.3:
         hi[:] = nbc - 1                       # along row 0
+    elif u < 0.6:
+        hi[:] = hi // 4                       # straight up, then along the last row
     return hi.astype(np.int32)
 
 
