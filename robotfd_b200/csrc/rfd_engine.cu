@@ -965,7 +965,7 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
     sh->mat = st->formula == 1;
   }
   __syncwarp();
-  w.cut0 = w.cut1 = -1;
+  w.cut = WalkCut{0, 0, 0};
   w.near_lo = 0;
   w.near_hi = -1;
   const bool pieces = g.size > 1 && sh->pd.recs;
@@ -980,8 +980,7 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
   if (band) {
     const int nbr = (sh->pd.n1 + 30) >> 5, nbc = (sh->pd.n2 + 30) >> 5;
     const int np = walk_pieces(sh->pd, g.size, nbr, nbc);
-    if (np > 1 && g.rank < np)
-      walk_cut(w, sh->pd, nbr, nbc, np, g.rank);
+    if (np > 1) walk_cut(w, sh->pd, nbr, nbc, np, g.rank);
     if (!walk_barrier(wa, g)) return false;  // (before a record changes)
   }
   // a radius to grow a level from: the larger of the endpoint bound and f x the points' spacing
@@ -1102,7 +1101,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) walk_kernel(WaveArgs wa, Walk
     return;
   }
   const int lane = threadIdx.x;
-  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, -1, -1, -1, 0, -1, 0};
+  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, -1, WalkCut{0, 0, 0}, 0, -1, 0};
   WalkGroup g;
   g.size = size;
   g.rank = blockIdx.x - group * size;

@@ -812,9 +812,9 @@ struct Walk {
   long long blocks;       // blocks swept
   int rec_from, rec_end;  // block rows whose records this sweep can be met at
   // where an earlier sweep's band ran: this member's piece, cut so that pieces take equal
-  // stretches of the band (cut0 < 0: equal block rows), and the chunks it entered it in (lo > hi:
-  // not known)
-  int cut0, cut1, near_lo, near_hi;
+  // stretches of the band, and the chunks it entered it in (lo > hi: not known)
+  WalkCut cut;
+  int near_lo, near_hi;
   int rounds;             // rounds of this phase's sweeps beyond each one's first two
 };
 
@@ -1158,10 +1158,15 @@ __device__ bool walk_start_row(const WaveArgs& wa, WalkShared* sh, Walk& w, int 
 }
 
 // The piece of member m by where the band of an earlier sweep ran, from the records (walk_cut_row;
-// the same for both its neighbours, since no record changes meanwhile).
+// the same for both its neighbours, since no record changes meanwhile).  Members past the last
+// piece only keep the number of pieces.
 __device__ void walk_cut(Walk& w, const PairDesc& pd, int nbr, int nbc, int pieces, int m) {
   const int lane = threadIdx.x & 31;
   const WalkRecord* recs = (const WalkRecord*)pd.recs;
+  w.cut = WalkCut{pieces, nbr, nbr};
+  w.near_lo = 0;
+  w.near_hi = -1;
+  if (m >= pieces) return;
   const int q = m + (lane & 1);  // lane 0: this piece's start, lane 1: its end
   const int row =
       q > 0 && q < pieces
@@ -1169,13 +1174,11 @@ __device__ void walk_cut(Walk& w, const PairDesc& pd, int nbr, int nbc, int piec
           : q > 0 ? nbr : 0;
   // (the band runs up and right, so these are in order; a long way along one row leaves pieces
   // without rows)
-  w.cut0 = __shfl_sync(kFull, row, 0);
-  w.cut1 = __shfl_sync(kFull, row, 1);
-  w.near_lo = 0;
-  w.near_hi = -1;
-  if (w.cut0 > 0) {
-    w.near_lo = __ldcg(&recs[w.cut0 - 1].lo);
-    w.near_hi = __ldcg(&recs[w.cut0 - 1].hi);
+  w.cut.row0 = __shfl_sync(kFull, row, 0);
+  w.cut.row1 = __shfl_sync(kFull, row, 1);
+  if (m > 0) {
+    w.near_lo = __ldcg(&recs[w.cut.row0 - 1].lo);
+    w.near_hi = __ldcg(&recs[w.cut.row0 - 1].hi);
   }
 }
 
@@ -1214,10 +1217,13 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
   // (members past the last piece only keep the barriers)
   const int pieces = walk_pieces(sh->pd, g.size, nbr, nbc);
   const int m = g.rank;
-  const bool cut = w.cut0 >= 0 && pieces > 1;
-  const int i0 = min(cut ? w.cut0 : (int)((long long)nbr * min(m, pieces) / pieces), nbr);
-  const int i1 = cut && m + 1 < pieces ? min(w.cut1, nbr)
-                                       : (int)((long long)nbr * min(m + 1, pieces) / pieces);
+  if (w.cut.pieces > 0 && w.cut.pieces != pieces) {
+    // cut for a grid of other pieces: again for this one, before a record changes
+    walk_cut(w, sh->pd, nbr, nbc, pieces, m);
+    if (!walk_barrier(wa, g)) return WALK_ERROR;
+  }
+  int i0, i1;
+  walk_piece(w.cut, m, pieces, nbr, &i0, &i1);
   WalkRecord* recs = reinterpret_cast<WalkRecord*>(sh->pd.recs);
   if (lane == 0) {
     sh->kind = KIND;
@@ -1366,7 +1372,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
       again = round == 0 || __ldcg(&st[before].changed);
       from = __ldcg(&st[before].which);
     }
-    if (done && rc == WALK_OK && res != none && m < pieces) {
+    if (done && rc == WALK_OK && res != none) {
       walk_cut(w, sh->pd, nbr, nbc, pieces, m);
       o.band = true;
     }

@@ -41,4 +41,26 @@ RFD_WHD int walk_cut_row(int q, int pieces, int n, int nbr, int nbc, Hi hi) {
   return a;
 }
 
+// A member's cut: rows row0 .. row1 - 1 of a grid cut in `pieces` (0: not cut yet).  Every member has
+// the same `pieces`, those past the last piece too.
+struct WalkCut {
+  int pieces, row0, row1;
+};
+
+// Block rows i0 .. i1 - 1 of piece m of a grid of nbr block rows (none for members past the last
+// piece).  A cut holds for its own number of pieces only - the DFD's grid, a row and a column
+// larger, can have one more than the VE-FD's - and otherwise all members take equal parts, so that
+// the pieces of a sweep always tile the grid.
+RFD_WHD void walk_piece(const WalkCut& c, int m, int pieces, int nbr, int* i0, int* i1) {
+  if (m >= pieces) {
+    *i0 = *i1 = nbr;
+  } else if (pieces > 1 && c.pieces == pieces) {
+    *i0 = c.row0;
+    *i1 = m + 1 < pieces ? c.row1 : nbr;
+  } else {
+    *i0 = (int)((long long)nbr * m / pieces);
+    *i1 = (int)((long long)nbr * (m + 1) / pieces);
+  }
+}
+
 }  // namespace rfd

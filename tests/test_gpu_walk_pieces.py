@@ -37,3 +37,13 @@ def test_band_far_along_the_first_row(ctx, strips, built, d, dwell, n, m):
     Q = np.concatenate([Q[0] + 0.01 * g.standard_normal((dwell, d)), Q])
     check(ctx, strips, P, Q)
     check(ctx, strips, Q, P)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("style,d,n1,n2", [
+    (0, 2, 449, 449), (0, 3, 609, 609), (1, 2, 929, 929), (0, 2, 1025, 850), (0, 2, 850, 1025),
+    (0, 2, 1889, 1600), (1, 3, 2049, 2049), (0, 2, 2049, 2049), (1, 3, 20001, 19003)])
+def test_grids_of_different_piece_counts(ctx, strips, built, style, d, n1, n2):
+    """Sizes whose DFD grid, a row and a column more than the VE-FD's, has a piece more."""
+    P, Q = built.gen_pair(style, d, n1, n2, 100.0 if style else 1.0, 0.1, 97, n1)
+    check(ctx, strips, P, Q)
