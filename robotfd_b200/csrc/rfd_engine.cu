@@ -2287,6 +2287,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   // even share of all blocks go first, in groups, and the others one CTA each.
   int wsize[2] = {1, 1};   // CTAs per group of the two plans
   int64_t wcount[2] = {0, 0};
+  bool walk_tail = false;  // the search's last pairs share the CTAs (walk, below)
   if (walks) {
     int* ho = (int*)(hbase + h_order);
     int* hp = (int*)(hbase + h_plan);
@@ -2303,6 +2304,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     if (lead) wsize[0] = (int)std::max<int64_t>(1, std::min(wg / lead, rows(0) / 2));
     wcount[0] = lead;
     wcount[1] = npairs - lead;
+    walk_tail = mode == MODE_DISTANCE && wcount[1] > 0;
     for (int s = 0; s < 2; ++s) {
       int* q = hp + (size_t)s * (2 + npairs);
       q[0] = (int)wcount[s];
@@ -2449,7 +2451,9 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       RFD_CUDA(cudaGetLastError());
       ++launches;
     }
-    if (walks && wsize[0] > 1) {
+    // (for every launch that can have groups: a plan's, or the search tail's, whose plan is made on
+    // the device)
+    if (walks && (wsize[0] > 1 || walk_tail)) {
       walk_ball_kernel<<<prep_grid(longest, npairs), 256, 0, st>>>(dt, (int)npairs);
       RFD_CUDA(cudaGetLastError());
       ++launches;
@@ -2514,7 +2518,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   // kWalkFirst probes of every pair; the few that need more then share the CTAs, twice.
   constexpr int kWalkFirst = 2, kWalkSecond = 8;
   auto walk = [&](int phases) -> int {
-    const bool tail = (phases & 4) && mode == MODE_DISTANCE && wcount[1] > 0;
+    const bool tail = (phases & 4) && walk_tail;
     int rc = walk_plans(phases, tail ? kWalkFirst : INT_MAX);
     for (int k = 0; k < 2 && tail && !rc; ++k) {
       walk_plan_kernel<<<1, 1024, 0, st>>>((const int*)(dbase + order_off), ds, (int)npairs,

@@ -47,3 +47,28 @@ def test_grids_of_different_piece_counts(ctx, strips, built, style, d, n1, n2):
     """Sizes whose DFD grid, a row and a column more than the VE-FD's, has a piece more."""
     P, Q = built.gen_pair(style, d, n1, n2, 100.0 if style else 1.0, 0.1, 97, n1)
     check(ctx, strips, P, Q)
+
+
+@pytest.mark.gpu
+def test_last_pairs_of_a_batch_of_like_pairs(strips, built):
+    """A batch without leading pairs, whose last ten searches share the CTAs: groups that start their
+    pieces by the chunks' bounds, in a workspace that an earlier call has filled.  (The curves lie
+    far from the origin, where zeros would say that no chunk is in reach.)"""
+    pairs = [built.gen_pair(0, 2, 900 + k % 7, 800 + k % 5, 1.0, 0.05, 98, k) for k in range(300)]
+    Ps, Qs = [p + 1000.0 for p, _ in pairs], [q + 1000.0 for _, q in pairs]
+    b = strips.distance_batch(Ps, Qs, precise=True)
+    d = np.array([r["distance"] for r in b])
+    wide = np.arange(300) % 30 == 0
+    brackets = np.stack([d * np.where(wide, 0.6, 1 - 1e-12), d * np.where(wide, 1.3, 1 + 1e-12)], axis=1)
+    c = built.Context(0)
+    try:
+        for fill in (0.0, 3.0):
+            big = [np.full((40000, 2), fill) + 1e-3 * np.arange(40000)[:, None] * (fill > 0)
+                   for _ in range(40)]
+            c.distance_batch(big[:20], big[20:], precise=True, max_probes=1)
+            for kw in (dict(brackets=brackets), dict(brackets=brackets, graph=True), dict()):
+                a = c.distance_batch(Ps, Qs, precise=True, **kw)
+                w = strips.distance_batch(Ps, Qs, precise=True, **{**kw, "graph": False})
+                assert [[x[k] for k in KEYS] for x in a] == [[x[k] for k in KEYS] for x in w]
+    finally:
+        c.close()
