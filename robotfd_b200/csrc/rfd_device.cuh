@@ -123,7 +123,7 @@ struct PairState {
   int kary_left;  // the pair: decisions of the round still running
   int kary_in;    // this decision belongs to a round
   int kary_reach; // its outcome
-  int walk_off;   // the walk gave the pair up: the strips take it
+  int walk_off;   // phases (bit 1 << phase) that the walk leaves to the strips
   int walk_band;  // the pair's records say where a walk's band ran
   double walk_ve; // VE-FD result a walk found ahead of the DFD (0: none)
   int corner;     // mirror decision: the far corner lies in the free space (see split_sync_kernel)

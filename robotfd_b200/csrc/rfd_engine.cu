@@ -901,8 +901,12 @@ struct WalkArgs {
   unsigned* ticket;
   int phases;              // 1 DFD, 2 VE-FD, 4 search
   int quota;               // probes per pair in this launch
-  // groups: arrival counts and announced pairs by group, reports and ends by CTA
+  int teams;               // of the strips' decisions on this device
+  float share;             // of the strips' time that a group may take: for a lone decision (< 1), or
+                           // for the first of a search
+  // groups: arrival counts, stop words and announced pairs by group, reports and ends by CTA
   unsigned* arrive;
+  unsigned* stop;
   int* next;               // [2][grid]
   WalkStat* stats;         // [2][grid]
   WalkEnd* ends;           // [3][grid]
@@ -932,8 +936,9 @@ __device__ __forceinline__ bool walk_skips_vefd(int quirks, const PairDesc& pd) 
 // read it again only after the next one: every phase passes at least one barrier before its
 // finalize, and one after it.
 // Returns false on an error (the error word is set).
+// npairs: pairs of the launch.
 __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh, Walk& w,
-                          WalkGroup& g, int p) {
+                          WalkGroup& g, int p, int npairs) {
   const int lane = threadIdx.x & 31;
   PairState* st = wa.st + p;
   const bool leader = g.rank == 0;
@@ -969,12 +974,30 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
   w.near_lo = 0;
   w.near_hi = -1;
   const bool pieces = g.size > 1 && sh->pd.recs;
-  // Rounds beyond the first two that a phase may take in all: a quarter of what the strips need
-  // for it (DFD 0.25 us a point, the others 7 us a strip or 3 us a chunk) at 10 us a round and
-  // 6 us a block row of a piece.
-  const double long_us = 3.0 / 32.0 * sh->pd.n1, round_us = 10.0 + 6.0 / 32.0 * sh->pd.n1 / g.size;
-  const int limit_dfd = 8 + (int)(0.25 * 0.25 * (sh->pd.n1 + sh->pd.n2) / round_us);
-  const int limit_dec = 8 + (int)(0.25 * fmax(long_us, 7.0 / 32.0 * sh->pd.n2) / round_us);
+  // The strips' time, in cycles: 7.5 us a strip and 3.5 a chunk of columns for the segment kinds
+  // (4,000 x 3,700 points 1.3 ms, 50,000 x 1,039 5.0, 300 x 260 0.1), 0.08 us a column and twice
+  // that a row for the DFD (fed strips).  Where the launch's pairs would fill the teams, a pair's
+  // turn there comes later by about half of that (150 pairs of 600 points: 5 times as long).
+  const PairDesc& in = wa.pairs[p];
+  const float S = (float)(in.n1 + 30) / 32.f, K = (float)(in.n2 + 30) / 32.f;
+  const float worth = fmaxf(1.f, 0.5f * (float)min(npairs, ka.teams) * S / (float)ka.teams);
+  const float strips_seg = worth * (20.f + 7.5f * S + 3.5f * K) * kWalkClock;
+  const float strips_dfd =
+      worth * (20.f + 0.08f * (float)(sh->pd.n1 + 2 * sh->pd.n2)) * kWalkClock;
+  // A phase begins: the share of the strips' time, and so many us more, that all its sweeps may take,
+  // and us a block ahead.  (A grid of a few blocks: as long as it takes.)
+  const bool few = (sh->pd.n1 + 30) / 32 + (sh->pd.n2 + 30) / 32 <= kWalkFew;
+  w.rule = g.size > 1 ? WALK_BY_TIME : npairs > 1 ? WALK_BY_EFFORT : WALK_BY_REST;
+  auto begin = [&](float strips, float share, float more, float pace) {
+    w.strips = few ? 1e12f : strips;
+    w.pace = few ? 0.f : pace * worth * kWalkClock;
+    w.deadline = clock64() + (long long)(share * w.strips + more * kWalkClock);
+    w.late = false;
+  };
+  const bool one_decision = ka.share < 1.f;
+  const float bound_share = ka.share > 1.5f ? 1.f : 0.55f, bound_pace = ka.share > 1.5f ? 0.f : 14.f;
+  // A search's decisions share their time: what one leaves of the strips' another may use.
+  float left = (ka.share - 1.f) * strips_seg;
   // Where an earlier launch's sweep found the band, pieces start from it.
   bool band = pieces && geti(&st->walk_band) != 0;
   if (band) {
@@ -991,7 +1014,7 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
   };
   for (int probes = 0;;) {
     const int phase = geti(&st->phase);
-    if (!geti(&st->active) || geti(&st->walk_off)) return true;
+    if (!geti(&st->active) || (geti(&st->walk_off) >> phase & 1)) return true;
     double res = 0.0;
     int rc = WALK_OK;
     if (phase == PH_DFD && (ka.phases & 1)) {
@@ -1001,13 +1024,14 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
       //
       // A group does the VE-FD first: its level can be so low that the band is a cell or two wide
       // and every piece meets its record at once, and the DFD's pieces then start near that band.
-      w.rounds = 0;
+      const bool ve_first = pieces && !walk_skips_vefd(geti(&st->quirks), sh->pd);
+      begin(ve_first ? strips_dfd + strips_seg : strips_dfd, bound_share, 100.f, bound_pace);
       double rad = first_radius(1.0);
-      if (pieces && !walk_skips_vefd(geti(&st->quirks), sh->pd)) {
+      if (ve_first) {
         double r = first_radius(0.5);
         for (int it = 0; it < 64; ++it, r *= 2.0) {
           const double level = __dmul_rn(r, r);
-          rc = walk_value<K_VEFD>(wa, sh, w, g, level, getd(&st->seed), limit_dec, band, res);
+          rc = walk_value<K_VEFD>(wa, sh, w, g, level, getd(&st->seed), band, res);
           if (rc != WALK_OK || res <= level) break;
         }
         if (rc == WALK_OK && res < kFltMax) {
@@ -1017,11 +1041,9 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
         if (rc == WALK_ERROR) return false;
         if (rc == WALK_GIVE_UP && !walk_barrier(wa, g)) return false;
       }
-      w.rounds = 0;
       for (int it = 0;; ++it, rad *= 2.0) {
         rc = it == 64 ? WALK_GIVE_UP
-                      : walk_value<K_DFD>(wa, sh, w, g, __dmul_rn(rad, rad), 0.0, limit_dfd, band,
-                                          res);
+                      : walk_value<K_DFD>(wa, sh, w, g, __dmul_rn(rad, rad), 0.0, band, res);
         if (rc != WALK_OK || res < kFltMax) break;
       }
       if (rc == WALK_OK && leader && lane == 0) {
@@ -1036,7 +1058,7 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
       // sooner the thinner the band is, so there the level grows up to the bound.
       const bool grow = geti(&st->coarse) != 0 || pieces;
       double rad = grow ? first_radius(0.5) : 0.0;
-      w.rounds = 0;
+      begin(strips_seg, bound_share, 100.f, bound_pace);
       for (;; rad *= 2.0) {
         if (ve > 0.0) {
           // (no sweep, so no barrier yet: the first member's finalize must not run ahead of the
@@ -1046,7 +1068,7 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
           break;
         }
         const double level = grow ? fmin(__dmul_rn(rad, rad), U) : U;
-        rc = walk_value<K_VEFD>(wa, sh, w, g, level, seed, limit_dec, band, res);
+        rc = walk_value<K_VEFD>(wa, sh, w, g, level, seed, band, res);
         if (rc != WALK_OK || res <= level || !(level < U)) break;
       }
       if (lane == 0 && sh->cells) atomicAdd(&st->cells_vefd, sh->cells);
@@ -1056,9 +1078,13 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
       }
     } else if (phase == PH_SEARCH && (ka.phases & 4) && probes < ka.quota) {
       ++probes;
-      w.rounds = 0;
-      WalkSweep o{false, INT_MAX, limit_dec, 0.0, false, false};
+      // a lone decision is given up as soon as it looks slow; a search's costs one of some thirty
+      if (one_decision) begin(strips_seg, ka.share, 80.f, 10.f);
+      else begin(strips_seg + left, 1.f, 0.f, 0.f);
+      const long long t0 = clock64();
+      WalkSweep o{false, INT_MAX, 0.0, false, false};
       rc = walk_sweep<K_DEC>(wa, sh, w, g, getd(&st->r2), getd(&st->split), 0.0, o, res);
+      left += strips_seg - (float)(clock64() - t0);
       if (lane == 0 && sh->cells) {
         atomicAdd(&st->cells_eval, sh->cells);
         atomicAdd(&st->cells_fp64, sh->cells64 / 2);
@@ -1073,7 +1099,8 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
     __syncwarp();
     if (lane == 0) {
       sh->cells = sh->cells64 = 0ull;
-      if (rc == WALK_GIVE_UP && leader) st->walk_off = 1;
+      if (rc == WALK_GIVE_UP && leader)
+        st->walk_off |= phase == PH_SEARCH ? 1 << PH_SEARCH : 1 << PH_DFD | 1 << PH_VEFD;
       if (leader && band) st->walk_band = 1;
     }
     if (rc == WALK_ERROR || !walk_barrier(wa, g)) return false;
@@ -1101,7 +1128,8 @@ __global__ void __launch_bounds__(kWalkThreads, 2) walk_kernel(WaveArgs wa, Walk
     return;
   }
   const int lane = threadIdx.x;
-  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, -1, WalkCut{0, 0, 0}, 0, -1, 0};
+  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, 0, -1, WalkCut{0, 0, 0}, 0, -1, WALK_BY_TIME, 0, 0.f, 0.f, false, 0u,
+         ka.stop + group};
   WalkGroup g;
   g.size = size;
   g.rank = blockIdx.x - group * size;
@@ -1122,7 +1150,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) walk_kernel(WaveArgs wa, Walk
       if (lane == 0) t = __ldcg(ka.next + (size_t)(turn & 1) * grid + group);
     }
     t = bcast(t);
-    if (t >= n || !walk_pair(wa, ka, sh, w, g, __ldg(ka.plan + 2 + t))) break;
+    if (t >= n || !walk_pair(wa, ka, sh, w, g, __ldg(ka.plan + 2 + t), n)) break;
   }
   walk_request(sh, w, kStop, 0);
 }
@@ -1139,7 +1167,8 @@ __global__ void __launch_bounds__(1024) walk_plan_kernel(const int* order, const
   for (int k0 = 0; k0 < npairs; k0 += 1024) {
     const int k = k0 + threadIdx.x;
     const int p = k < npairs ? order[k] : 0;
-    const bool in = k < npairs && st[p].active && st[p].phase == phase && !st[p].walk_off;
+    const bool in = k < npairs && st[p].active && st[p].phase == phase &&
+                    !(st[p].walk_off >> phase & 1);
     const unsigned b = __ballot_sync(kFull, in);
     if (lane == 0) warp_n[warp] = __popc(b);
     __syncthreads();
@@ -1842,6 +1871,14 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     const int64_t hi = std::max(n1s[p], n2s[p]), lo = std::min(n1s[p], n2s[p]);
     return walks && hi >= kWalkAspectFrom && hi >= kWalkAspect * lo;
   };
+  // Phases of a pair (bit 1 << phase) that the walk leaves to the strips from the start: all of a thin
+  // pair's, and a lone decision on a grid of up to three pieces (600 x 610 points: 0.36 ms on the
+  // strips, 0.23 to 0.28 walked where the band is thin, 0.55 where it is not).
+  auto walk_blocks = [&](int64_t p) { return (n1s[p] + 30) / 32 + (n2s[p] + 30) / 32; };
+  auto walk_off = [&](int64_t p) -> int {
+    if (thin(p)) return 1 << PH_DFD | 1 << PH_VEFD | 1 << PH_SEARCH;
+    return mode == MODE_DECIDE && walk_blocks(p) < 4 * kWalkStretch ? 1 << PH_SEARCH : 0;
+  };
   auto tree_fits = [&](int64_t p) {
     return thin(p) && n1s[p] >= 2 && n2s[p] >= 2 && (trows(p) - 1 + 31) / 32 * 3 <= ctx->team_grid[K_DEC] * 5 / 4;
   };
@@ -1969,7 +2006,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   L.zero_begin = off;
   // the walk's ticket counters and groups' arrival counts, a set per launch
   constexpr int kWalkLaunches = 8;
-  const size_t walk_ticket = take(sizeof(unsigned) * kWalkLaunches * (1 + wg));
+  const size_t walk_ticket = take(sizeof(unsigned) * kWalkLaunches * (1 + 2 * wg));
   L.counters = take(sizeof(unsigned) * (wbase + wtickets));
   const size_t prof_off = take(sizeof(unsigned long long) * (kTraceBase + kTraceW * kTrace));
   L.error = take(sizeof(int));
@@ -2189,7 +2226,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     s.blo = s.bhi = NAN;
     s.coarse = (ck && n1 >= 2 && n2 >= 2) ? 1 : 0;
     s.formula = formula[p];
-    s.walk_off = thin(p);
+    s.walk_off = walk_off(p);
     if (o.bracket && mode == MODE_DISTANCE) {
       s.blo = o.bracket[2 * p];
       s.bhi = o.bracket[2 * p + 1];
@@ -2288,6 +2325,10 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   int wsize[2] = {1, 1};   // CTAs per group of the two plans
   int64_t wcount[2] = {0, 0};
   bool walk_tail = false;  // the search's last pairs share the CTAs (walk, below)
+  // Calls that the walk has nothing to do for; and calls of small pairs, grids of one or two pieces
+  // but more than a few blocks, whose DFD and VE-FD start on the strips: chains of a few strips
+  // there (bounds of 300 x 260 points 0.41 ms, 0.40 to 0.53 walked, 2.0 where the band is wide).
+  bool walk_none = true, walk_small = mode != MODE_DECIDE && 2 * npairs <= wg, few = true;
   if (walks) {
     int* ho = (int*)(hbase + h_order);
     int* hp = (int*)(hbase + h_plan);
@@ -2305,6 +2346,12 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     wcount[0] = lead;
     wcount[1] = npairs - lead;
     walk_tail = mode == MODE_DISTANCE && wcount[1] > 0;
+    for (int64_t p = 0; p < npairs; ++p) {
+      walk_none = walk_none && (walk_off(p) >> PH_SEARCH & 1);
+      walk_small = walk_small && walk_blocks(p) < 3 * kWalkStretch;
+      few = few && walk_blocks(p) <= kWalkFew;
+    }
+    walk_small = walk_small && !few;
     for (int s = 0; s < 2; ++s) {
       int* q = hp + (size_t)s * (2 + npairs);
       q[0] = (int)wcount[s];
@@ -2416,7 +2463,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
                              cudaMemcpyHostToDevice, st));
     RFD_CUDA(cudaMemcpyAsync(dbase + L.titems, hbase + L.h_titems, sizeof(int2) * ntitems,
                              cudaMemcpyHostToDevice, st));
-    if (walks) {
+    if (walks && !walk_none) {
       RFD_CUDA(cudaMemcpyAsync(dbase + order_off, hbase + h_order, sizeof(int) * npairs,
                                cudaMemcpyHostToDevice, st));
       RFD_CUDA(cudaMemcpyAsync(dbase + plan_off, hbase + h_plan, sizeof(int) * (2 + npairs) * 2,
@@ -2453,7 +2500,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     }
     // (for every launch that can have groups: a plan's, or the search tail's, whose plan is made on
     // the device)
-    if (walks && (wsize[0] > 1 || walk_tail)) {
+    if (walks && !walk_none && (wsize[0] > 1 || walk_tail)) {
       walk_ball_kernel<<<prep_grid(longest, npairs), 256, 0, st>>>(dt, (int)npairs);
       RFD_CUDA(cudaGetLastError());
       ++launches;
@@ -2486,10 +2533,13 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   auto walk_launch = [&](int plan, bool groups, int64_t ctas, int phases, int quota) -> int {
     WalkArgs ka{};
     ka.plan = (const int*)(dbase + plan_off) + (size_t)plan * (2 + npairs);
-    ka.ticket = (unsigned*)(dbase + walk_ticket) + (size_t)nwalk * (1 + wg);
+    ka.ticket = (unsigned*)(dbase + walk_ticket) + (size_t)nwalk * (1 + 2 * wg);
     ka.arrive = ka.ticket + 1;
+    ka.stop = ka.arrive + wg;
     ka.phases = phases;
     ka.quota = quota;
+    ka.teams = ctx->team_grid[K_DEC];
+    ka.share = mode == MODE_DECIDE ? 0.25f : npairs > 1 ? 2.f : 1.3f;
     ka.next = (int*)(dbase + wnext_off);
     ka.stats = (WalkStat*)(dbase + wstat_off);
     ka.ends = (WalkEnd*)(dbase + wend_off);
@@ -2793,7 +2843,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   auto issue = [&]() -> int {
     int rc = upload();
     if (rc) return rc;
-    if (!walks) {
+    if (!walks || walk_none) {
       rc = strips(mode == MODE_DECIDE ? 4 : 7);
       return rc ? rc : read_back();
     }
@@ -2807,6 +2857,15 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     int dfd = ck || wcount[1] > 0 ? 0 : 1;
     for (int64_t p = 0; p < npairs && dfd; ++p)
       if (std::max(n1s[p], n2s[p]) >= kWalkAspect * std::min(n1s[p], n2s[p])) dfd = 0;
+    if (walk_small && search) {
+      rc = strips(3);
+      if (rc) return rc;
+      if (ctx->timing) RFD_CUDA(record(2));
+      if (mode == MODE_DISTANCE) rc = walk(4);
+      if (rc) return rc;
+      if (ctx->timing) RFD_CUDA(record(3));
+      return read_back();
+    }
     if (!dfd && mode != MODE_DECIDE) {
       rc = strips(1);
       if (rc) return rc;
@@ -2901,17 +2960,41 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   }
   RFD_CUDA(cudaStreamSynchronize(st));
   if (walks && hmisc[1] == 0) {
-    // what the walk gave up, from the phase it was in (bit 1 << phase), on the strips
-    unsigned open = 0;
-    for (int64_t p = 0; p < npairs; ++p)
-      if (hs[p].phase != PH_DONE) open |= 1u << hs[p].phase;
-    if (open) {
-      const int parts = ((open >> PH_DFD) & 1) | (open & ~(1u << PH_SEARCH) ? 2 : 0) | 4;
+    // What the walk left, from the phase it was in (bit 1 << phase), on the strips: up to the search
+    // first, which the walk takes where it can, then the searches that it has given up.
+    auto open = [&](bool walkable) {
+      unsigned m = 0;
+      for (int64_t p = 0; p < npairs; ++p)
+        if (hs[p].phase != PH_DONE && !(walkable && (hs[p].walk_off >> PH_SEARCH & 1)))
+          m |= 1u << hs[p].phase;
+      return m;
+    };
+    auto pass = [&](int parts, bool walk_search) -> int {
       RFD_CUDA(cudaMemsetAsync(dbase + L.zero_begin, 0, L.zero_end - L.zero_begin, st));
       int rc2 = strips(parts);
-      if (!rc2) rc2 = read_back();
+      if (rc2) return rc2;
+      if (walk_search) {
+        if (ctx->timing) RFD_CUDA(record(2));
+        nwalk = 0;
+        rc2 = walk(4);
+        if (rc2) return rc2;
+        if (ctx->timing) RFD_CUDA(record(3));
+      }
+      rc2 = read_back();
       if (rc2) return rc2;
       RFD_CUDA(cudaStreamSynchronize(st));
+      return RFD_OK;
+    };
+    const unsigned before = ~(1u << PH_SEARCH);
+    const unsigned o1 = open(false);
+    if (o1 & before) {
+      const bool ws = mode == MODE_DISTANCE && (open(true) & before) != 0;
+      const int rc2 = pass((int)(o1 >> PH_DFD & 1) | 2 | (ws ? 0 : 4), ws);
+      if (rc2) return rc2;
+    }
+    if (hmisc[1] == 0 && open(false)) {
+      const int rc2 = pass(4, false);
+      if (rc2) return rc2;
     }
   }
   if (guard) {
@@ -3831,8 +3914,14 @@ extern "C" int32_t rfd_decide_noalloc(const double* c1, int64_t n1, const double
   ka.ticket = (unsigned*)(base + o_walk);
   ka.phases = 4;
   ka.quota = 1;
-  walk_kernel<<<1, kWalkThreads, kWalkSmem, st>>>(wa, ka);
-  RFD_CUDA(cudaGetLastError());
+  ka.teams = nd.team_grid;
+  // (no walk on grids below kWalkLeast blocks, rows and columns together: 150 x 140 points take 100 us
+  // on the strips, 75 to 100 with the walk, 200 where the band is wide)
+  constexpr int64_t kWalkLeast = 16;
+  if ((n1 + 30) / 32 + (n2 + 30) / 32 >= kWalkLeast) {
+    walk_kernel<<<1, kWalkThreads, kWalkSmem, st>>>(wa, ka);
+    RFD_CUDA(cudaGetLastError());
+  }
   bnd_fill_kernel<<<dim3(256, 1), 256, 0, st>>>(ddesc, dstate, 1, PH_SEARCH, nullptr, nullptr, 0, 0);
   RFD_CUDA(cudaGetLastError());
   team_kernel<K_DEC, 8><<<nd.team_grid, kTeamThreads, team_smem_bytes<K_DEC>(), st>>>(wa);

@@ -38,8 +38,9 @@
 // piece that ends empty from everything that could be live ends the sweep (walk_sweep).  Once a
 // sweep has found the band, the next ones start their pieces only near where it ran.
 //
-// A sweep whose band is not thin (list overflow, effort against progress) gives up; the pair's
-// phase then runs on the strips as before.
+// A sweep whose band is not thin (list overflow, time against progress) gives up, and so does a
+// phase past a share of the strips' time (walk_slow, walk_pair); the pair's phase then runs on the
+// strips.
 //
 // What bounds it: the chain of a band's blocks.  A decision's block takes about 5,300 cycles (the
 // rows 2,900, waiting for the tile 900, the next block's choice 500; a tile is ready 3,500 after
@@ -72,6 +73,7 @@ constexpr int kWalkVals = 2048;
 // A block row's output list as recorded by the first walk of a piece (n < 0: too long to record),
 // and the chunks lo .. hi of the list as last walked.
 constexpr int kWalkRec = 4;
+constexpr float kWalkClock = 1900.f;  // cycles a microsecond, about
 struct WalkRecord {
   int n, lo, hi, pad;
   int j[kWalkRec];
@@ -90,6 +92,9 @@ struct WalkStat {
   double c, res;
   int changed, which, empty, part, gave_up, skip;
 };
+// WalkStat::gave_up: the piece ends the phase; past the phase's deadline; the first walk, from what
+// could be live, was given up (the piece is left to the rounds).
+constexpr int kGaveUp = 1, kLate = 2, kCrowded = 4;
 // Points 32 J .. 32 J + 32 of a curve within rad of the centre (rad infinite: no bound).
 struct WalkBall {
   double x[3], rad;
@@ -809,19 +814,62 @@ struct Walk {
   unsigned seq_p, seq_c;  // tiles requested, taken
   int pi, pj;             // the outstanding request (pi < 0: none)
   int cur, n;             // list of the row below: buffer and live chunks
-  long long blocks;       // blocks swept
+  long long t0;           // cycle the running walk began
+  int blocks;             // its blocks and listed edges (256 count as a block)
   int rec_from, rec_end;  // block rows whose records this sweep can be met at
   // where an earlier sweep's band ran: this member's piece, cut so that pieces take equal
   // stretches of the band, and the chunks it entered it in (lo > hi: not known)
   WalkCut cut;
   int near_lo, near_hi;
-  int rounds;             // rounds of this phase's sweeps beyond each one's first two
+  // of the phase (walk_pair): its rule of giving up, cycle past which it is given up, cycles that the
+  // strips would need, cycles that a piece may take for a block ahead (0: any); whether the
+  // deadline has passed (the same for all members)
+  int rule;
+  long long deadline;
+  float strips, pace;
+  bool late;
+  // the group's sweeps so far, and its word that holds the number of the last one whose end was
+  // known before every piece had been walked
+  unsigned sweeps;
+  unsigned* stop;
 };
 
-enum WalkStatus : int { WALK_OK = 0, WALK_ERROR, WALK_GIVE_UP, WALK_MET, WALK_UNSETTLED };
+enum WalkStatus : int { WALK_OK = 0, WALK_ERROR, WALK_GIVE_UP, WALK_MET, WALK_UNSETTLED, WALK_STOPPED };
 // How a piece is walked: alone (the whole grid); the first time from what could be live, or
 // from the true start, recording every block row's list; again, until it meets a record.
 enum WalkMode : int { WALK_ALONE = 0, WALK_RECORD = 1, WALK_AGAIN = 2 };
+
+// Rules of giving up (walk_slow), by what the strips would cost instead:
+//   WALK_BY_EFFORT  blocks and listed edges against the blocks the walk has come ahead: a thin band
+//                   lists a few hundred edges a block and goes from block to block right or up (a
+//                   pair of many, each walked by one CTA: the strips' time is the call's then);
+//   WALK_BY_REST    a lone CTA's walk, once a twelfth of the strips' time has passed (60 us at
+//                   most): if the rest at this rate takes longer than the strips (what is spent is
+//                   spent; 1.15: rates vary along a band);
+//   WALK_BY_TIME    a group's: the phase's deadline; and a piece, where `pace` says so, against a thin
+//                   band's rate, which is about 5 us a block row or column for the decision and 8
+//                   for the others.  A wide band's blocks cost 16 us and more (all of their edges
+//                   listed), and nothing says that before they are walked.
+enum WalkRule : int { WALK_BY_EFFORT = 0, WALK_BY_REST, WALK_BY_TIME };
+__device__ __forceinline__ bool walk_slow(const Walk& w, int ahead, int total) {
+  if (w.rule == WALK_BY_EFFORT) return w.blocks > 64 + 4LL * (ahead - 1);
+  constexpr float us = kWalkClock;
+  const long long now = clock64();
+  const float spent = (float)(now - w.t0);
+  bool slow;
+  if (w.rule == WALK_BY_REST)
+    slow = spent > fminf(w.strips / 12.f, 60.f * us) &&
+           spent * (float)(total - ahead) > 1.15f * w.strips * (float)ahead;
+  else
+    slow = now > w.deadline ||
+           (w.pace > 0.f && spent > fmaxf(15.f * us + w.pace * (float)ahead, 0.12f * w.strips));
+  return bcast((int)slow) != 0;
+}
+// Tells the other members that this sweep's end is known, or that it is given up.
+__device__ __forceinline__ void walk_stop(const Walk& w) {
+  if ((threadIdx.x & 31) == 0) *(volatile unsigned*)w.stop = w.sweeps;
+  __syncwarp();
+}
 
 __device__ __forceinline__ void walk_request(WalkShared* sh, Walk& w, int i, int j) {
   if ((threadIdx.x & 31) == 0) {
@@ -932,14 +980,18 @@ __device__ int walk_rows(const WaveArgs& wa, WalkShared* sh, Walk& w, int i0, in
       double F = upv[lane];
       unsigned V = __ballot_sync(kFull, walk_live<KIND>(F));
       k += have;
+      // (on its way while the tile is waited for)
+      const unsigned stop = mode != WALK_ALONE ? *(volatile unsigned*)w.stop : 0u;
       const int slot = walk_get(wa, sh, w, i, j);
       if (slot < 0) { status = WALK_ERROR; break; }
-      // effort against progress: a thin band lists a few hundred edges a block and goes from block
-      // to block right or up
-      w.blocks += 1 + (sh->cnt[slot] >> 8);
       j_min = min(j_min, j);
       j_max = max(j_max, j);
-      if (w.blocks > 64 + 4LL * ((i - i0) + (j_max - j_min)) || (on == kWalkCap && !loose)) {
+      w.blocks += 1 + (sh->cnt[slot] >> 8);
+      if (mode != WALK_ALONE && bcast(stop) == w.sweeps) {
+        status = WALK_STOPPED;
+        break;
+      }
+      if (walk_slow(w, (i - i0) + (j_max - j_min) + 1, nbr + nbc) || (on == kWalkCap && !loose)) {
         status = WALK_GIVE_UP;
         break;
       }
@@ -1193,7 +1245,6 @@ __device__ __forceinline__ int walk_pieces(const PairDesc& pd, int size, int nbr
 struct WalkSweep {
   bool flat;
   int rounds;
-  int limit;  // of Walk::rounds: past it the phase is given up
   // out: the largest of the least values the pieces end with.  No path has less if the pieces
   // started from everything that could be live (sure).
   double least;
@@ -1234,6 +1285,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
   sh->dead_row[lane] = dead;
   w.cur = 0;
   w.n = 0;
+  w.t0 = clock64();
   w.blocks = 0;
   w.rec_from = 0;
   w.rec_end = -1;
@@ -1255,21 +1307,29 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
   if (pieces == 1) {
     int rc = WALK_OK;
     if (m == 0) rc = walk_rows<KIND>(wa, sh, w, 0, nbr, start, res, WALK_ALONE, nullptr, false, lost, c);
-    if (g.size == 1) return rc;
+    const int late = bcast(w.rule == WALK_BY_TIME && clock64() > w.deadline ? kLate : 0);
+    if (g.size == 1) {
+      w.late = late != 0;
+      return rc;
+    }
     if (rc == WALK_ERROR) return rc;
     if (m == 0 && lane == 0) {
       WalkStat* q = g.stat[0] + g.first;
       __stcg(&q->res, res);
-      __stcg(&q->gave_up, (int)(rc == WALK_GIVE_UP));
+      __stcg(&q->gave_up, (rc == WALK_GIVE_UP ? kGaveUp : 0) | late);
     }
     if (!walk_barrier(wa, g)) return WALK_ERROR;
     const WalkStat* q = g.stat[0] + g.first;
+    const int up = __ldcg(&q->gave_up);
     res = __ldcg(&q->res);
-    return __ldcg(&q->gave_up) ? WALK_GIVE_UP : WALK_OK;
+    w.late = (up & kLate) != 0;
+    return up & kGaveUp ? WALK_GIVE_UP : WALK_OK;
   }
+  ++w.sweeps;
   const bool on = m < pieces && i0 < i1;
   WalkStat me{0.0, none, on, 0, 0, 0, 0, !on};
   auto report = [&](int round) {
+    if (clock64() > w.deadline) me.gave_up |= kLate;
     if (m < pieces && lane == 0) {
       WalkStat* q = g.stat[round & 1] + g.first + m;
       __stcg(&q->c, me.c);
@@ -1290,16 +1350,18 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     int rc = WALK_OK;
     if (!err) rc = walk_rows<KIND>(wa, sh, w, i0, i1, start, me.res, WALK_RECORD, recs, m > 0, lost, c);
     if (err || rc == WALK_ERROR) return WALK_ERROR;
-    if (rc == WALK_GIVE_UP) {
-      if (m == 0) me.gave_up = 1;
+    if (rc == WALK_GIVE_UP || rc == WALK_STOPPED) {
+      if (rc == WALK_GIVE_UP) me.gave_up = m == 0 ? kGaveUp : kCrowded;
+      if (me.gave_up == kGaveUp) walk_stop(w);
       lost = true;  // (a start from too much: the piece is left to the rounds)
       w.n = 0;
       w.rec_end = -1;
     }
     walk_save_end(sh, w, g.end[0] + g.first + m);
-    first_empty = me.empty = w.n == 0 && i1 < nbr;
+    first_empty = me.empty = rc != WALK_STOPPED && w.n == 0 && i1 < nbr;
     first_res = me.res;
     me.part = lost;
+    if (me.empty && (m == 0 || !lost)) walk_stop(w);
     if (KIND != K_DEC && w.rec_end >= 0) {
       // the least value the piece ends with, in place of the constant in this report
       double v = i1 == nbr ? me.res : dead;
@@ -1315,13 +1377,16 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     // the round's reports
     const WalkStat* st = g.stat[round & 1] + g.first;
     int moved = INT_MAX, bad = 0, hollow = INT_MAX, hollow_all = 0, part = 0, end = 0;
+    int crowd = 0;  // pieces left to the rounds: 2 each, against one for each piece
     double cc = 0.0;
     for (int q = lane; q < pieces; q += 32) {
       const WalkStat* s = st + q;
       if (__ldcg(&s->skip)) continue;
       end = q;
       const int empty = __ldcg(&s->empty);
-      bad |= __ldcg(&s->gave_up);
+      const int up = __ldcg(&s->gave_up);
+      bad |= up;
+      crowd += (up & kCrowded ? 2 : 0) - 1;
       if (round > 0 && __ldcg(&s->changed)) moved = min(moved, q);
       if (empty) hollow = min(hollow, q);
       const int lossy = __ldcg(&s->part);
@@ -1334,6 +1399,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
       moved = min(moved, __shfl_xor_sync(kFull, moved, d));
       hollow = min(hollow, __shfl_xor_sync(kFull, hollow, d));
       bad |= __shfl_xor_sync(kFull, bad, d);
+      crowd += __shfl_xor_sync(kFull, crowd, d);
       hollow_all |= __shfl_xor_sync(kFull, hollow_all, d);
       part |= __shfl_xor_sync(kFull, part, d);
       end = max(end, __shfl_xor_sync(kFull, end, d));
@@ -1341,7 +1407,8 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     }
     const double last = __ldcg(&st[end].res);
     int done = 0, rc = WALK_OK;
-    if (bad) {
+    w.late = (bad & kLate) != 0;
+    if (bad & kGaveUp) {
       done = 1;
       rc = WALK_GIVE_UP;
     } else if (round == 0) {
@@ -1361,7 +1428,8 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
       done = 1;
       rc = WALK_UNSETTLED;
     }
-    if (!done && round > 1 && ++w.rounds > o.limit) {
+    // (of more than half of the pieces left to the rounds some follow one another)
+    if ((!done || rc == WALK_UNSETTLED) && (w.late || (w.pace > 0.f && round == 0 && crowd > 0))) {
       done = 1;
       rc = WALK_GIVE_UP;
     }
@@ -1381,13 +1449,15 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     me.changed = 0;
     if (again) {
       walk_load_end(sh, w, g.end[from] + g.first + before);
+      w.t0 = clock64();
       w.blocks = 0;
       c = 0.0;
       double r = none;
       int q = WALK_OK;
       if (w.n) q = walk_rows<KIND>(wa, sh, w, i0, i1, dead, r, WALK_AGAIN, recs, false, lost, c);
       if (q == WALK_ERROR) return WALK_ERROR;
-      me.gave_up = q == WALK_GIVE_UP;
+      me.gave_up = q == WALK_GIVE_UP ? kGaveUp : 0;
+      if (me.gave_up) walk_stop(w);
       if (q == WALK_MET) {
         me.which = 0;
         me.c = c;
@@ -1414,13 +1484,15 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
 // it, and none survives the next smaller number.
 template <int KIND>
 __device__ int walk_value(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup& g, double level,
-                          double seed, int limit, bool& band, double& res) {
+                          double seed, bool& band, double& res) {
   constexpr int kRounds = 3;
   int rc = WALK_OK;
   // one sweep and the barrier after it; true when the caller goes on with `out`
   double out = kFltMax;
-  WalkSweep o{false, kRounds, limit, 0.0, false, false};
+  WalkSweep o{false, kRounds, 0.0, false, false};
   auto sweep = [&](bool flat, int rounds, double at) -> bool {
+    rc = WALK_GIVE_UP;
+    if (w.late) return false;
     o.flat = flat;
     o.rounds = rounds;
     rc = walk_sweep<KIND>(wa, sh, w, g, at, sqrt(at), seed, o, out);

@@ -14,6 +14,7 @@ namespace rfd {
 // of at least kWalkStretch blocks of a thin band (shorter ones end before the band has forgotten
 // their start).
 constexpr int kWalkStretch = 10;
+constexpr int kWalkFew = 6;  // a grid of a few blocks: at most so many, rows and columns together
 RFD_WHD int walk_pieces(int size, int nbr, int nbc) {
   int n = size < nbr / 2 ? size : nbr / 2;
   const int by_length = (nbr + nbc) / kWalkStretch;
