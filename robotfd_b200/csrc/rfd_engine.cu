@@ -1483,7 +1483,9 @@ struct rfd_context {
   int search_window = 2;  // continuous search: strips a probe queues ahead of its band
   int dfd_rows = 8;    // rows per lane of the DFD strips (RFD_DFD_ROWS = 1, 2, 4 or 8)
   int dfd_auto = 1;    // neither set by RFD_DFD_ROWS nor tuned
-  int dfd_skew = -1;   // RFD_DFD_SKEW: 1 skewed rows, 0 stacked, unset: chosen per call
+  int dfd_skew = -1;   // RFD_DFD_SKEW or tuned: 1 skewed rows, 0 stacked, unset: chosen per call
+  int dfd_fed = 1;     // fed strips where they are few (not with RFD_DFD_SKEW)
+  int tuning = 0;      // an autotuner's call: 1 no walk, 2 no fed strips (what it times must run)
   int dfd_grid[2] = {0, 0};  // [stacked, skewed] for dfd_rows
   int dfd_grid_all[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};  // for rows 1, 2, 4, 8
   int fed_grid[2] = {0, 0};  // fed strips: plain, inflated
@@ -1866,7 +1868,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
   constexpr int kWalkAspect = 8, kWalkAspectFrom = 8192;
   // Without search_arity, tree rounds (tree_arm): for the pairs that stay on the strips as long and thin
   // ones, where two probes' worth of other strips fit beside a pair's own.
-  const bool walks = ctx->walk && !o.dense && !ctx->solo && !ctx->prof;
+  const bool walks = ctx->walk && !o.dense && !ctx->solo && !ctx->prof && !(ctx->tuning & 1);
   auto thin = [&](int64_t p) {
     const int64_t hi = std::max(n1s[p], n2s[p]), lo = std::min(n1s[p], n2s[p]);
     return walks && hi >= kWalkAspectFrom && hi >= kWalkAspect * lo;
@@ -2690,7 +2692,7 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
         const int64_t r = ck && n1s[p] >= 2 && n2s[p] >= 2 ? coarse_n(n1s[p]) : turn ? trows(p) : n1s[p];
         fstrips += (r + 31) / 32;
       }
-      const bool fed = ctx->dfd_skew < 0 && fstrips <= (int64_t)ctx->fed_grid[ck > 0] * kFedTeams;
+      const bool fed = ctx->dfd_fed && !(ctx->tuning & 2) && fstrips <= (int64_t)ctx->fed_grid[ck > 0] * kFedTeams;
       if (fed && turn) ddfd = dt;
       // Batches: four stacked rows a lane while the strips of eight are at most ten times the
       // resident warps (the long pairs' strips, a chain, then end sooner: 1,024 uneven pairs
@@ -3248,7 +3250,7 @@ int32_t rfd_context_create(int32_t device, rfd_context** out) {
     if (dr && (dr[0] == '1' || dr[0] == '2' || dr[0] == '4' || dr[0] == '8') && !dr[1])
       c->dfd_rows = dr[0] - '0', c->dfd_auto = 0;
     const char* dk = getenv("RFD_DFD_SKEW");
-    if (dk && (dk[0] == '0' || dk[0] == '1') && !dk[1]) c->dfd_skew = dk[0] - '0';
+    if (dk && (dk[0] == '0' || dk[0] == '1') && !dk[1]) c->dfd_skew = dk[0] - '0', c->dfd_fed = 0;
     for (int ri = 0; ri < 4; ++ri)
       for (int sk = 0; sk < 2; ++sk) {
         int od = 0;
@@ -3439,8 +3441,9 @@ int32_t rfd_distance_batch(rfd_context* ctx, int64_t npairs, const double* const
 // Autotuner of the DFD sweep's tile shape: rows per lane (the strip height, 32 x 1, 2, 4 or 8)
 // and the layout of a lane's rows (stacked: fewer instructions per cell; skewed: independent
 // cells per step).  Each candidate sweeps the caller's pairs `reps` times (CUDA-event phase
-// times of rfd_bounds-style calls); the fastest is kept in the context for later calls, which
-// otherwise use 8 rows and choose the layout by strip count.
+// times of rfd_bounds-style calls on the strips: no walk, no fed strips, which these shapes do not
+// touch); the fastest is kept in the context for later calls' strips that are not fed, which
+// otherwise use 4 or 8 rows and choose the layout by strip count.
 int32_t rfd_autotune(rfd_context* ctx, int64_t npairs, const double* const* c1s, const int64_t* n1s,
                      const double* const* c2s, const int64_t* n2s, const int32_t* dims,
                      const rfd_options* opt, int32_t reps, double* ms_out, int32_t* best_out) {
@@ -3460,6 +3463,7 @@ int32_t rfd_autotune(rfd_context* ctx, int64_t npairs, const double* const* c1s,
   double best = 1e300;
   int best_r = keep_rows, best_s = keep_skew;
   int rc = RFD_OK;
+  ctx->tuning = 3;
   for (int ri = 0; ri < 4 && rc == RFD_OK; ++ri)
     for (int sk = 0; sk < 2 && rc == RFD_OK; ++sk) {
       ctx->dfd_rows = rows[ri];
@@ -3481,6 +3485,7 @@ int32_t rfd_autotune(rfd_context* ctx, int64_t npairs, const double* const* c1s,
         best_s = sk;
       }
     }
+  ctx->tuning = 0;
   ctx->dfd_rows = rc == RFD_OK ? best_r : keep_rows;
   ctx->dfd_skew = rc == RFD_OK ? best_s : keep_skew;
   const int bi = ctx->dfd_rows == 1 ? 0 : ctx->dfd_rows == 2 ? 1 : ctx->dfd_rows == 4 ? 2 : 3;
@@ -3500,7 +3505,8 @@ int32_t rfd_autotune(rfd_context* ctx, int64_t npairs, const double* const* c1s,
 // helpers), the switch point (active pairs below which the continuous search takes over: a
 // quarter of the team count, the team count, or every pair from the first probe) and the start window (strips a probe queues ahead: 1, 2,
 // 4).  Each candidate solves the caller's pairs once untimed and `reps` times timed (CUDA-event
-// phase times of whole solves with the caller's options); the fastest is kept in the context.
+// phase times of whole solves with the caller's options, on the strips: no walk); the fastest is kept
+// in the context.
 int32_t rfd_autotune_search(rfd_context* ctx, int64_t npairs, const double* const* c1s,
                             const int64_t* n1s, const double* const* c2s, const int64_t* n2s,
                             const int32_t* dims, const rfd_options* opt, int32_t reps,
@@ -3521,6 +3527,7 @@ int32_t rfd_autotune_search(rfd_context* ctx, int64_t npairs, const double* cons
   const int warps[2] = {4, 8}, windows[3] = {1, 2, 4};
   double best = 1e300;
   int bw = keep_w, bs = keep_sw, bn = keep_win, rc = RFD_OK;
+  ctx->tuning = 1;
   for (int wi = 0; wi < 2 && rc == RFD_OK; ++wi)
     for (int si = 0; si < 3 && rc == RFD_OK; ++si)
       for (int ni = 0; ni < 3 && rc == RFD_OK; ++ni) {
@@ -3543,6 +3550,7 @@ int32_t rfd_autotune_search(rfd_context* ctx, int64_t npairs, const double* cons
           bn = windows[ni];
         }
       }
+  ctx->tuning = 0;
   ctx->team_warps = rc == RFD_OK ? bw : keep_w;
   for (int k = 0; k < 3; ++k) ctx->team_grid[k] = ctx->team_grids[team_shape_index(ctx->team_warps)][k];
   ctx->search_switch = rc == RFD_OK ? bs : keep_sw;
