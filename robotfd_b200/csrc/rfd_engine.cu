@@ -980,7 +980,8 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
   // turn there comes later by about half of that (150 pairs of 600 points: 5 times as long).
   const PairDesc& in = wa.pairs[p];
   const float S = (float)(in.n1 + 30) / 32.f, K = (float)(in.n2 + 30) / 32.f;
-  const float worth = fmaxf(1.f, 0.5f * (float)min(npairs, ka.teams) * S / (float)ka.teams);
+  const float worth =
+      npairs > 1 ? fmaxf(1.f, 0.5f * (float)min(npairs, ka.teams) * S / (float)ka.teams) : 1.f;
   const float strips_seg = worth * (20.f + 7.5f * S + 3.5f * K) * kWalkClock;
   const float strips_dfd =
       worth * (20.f + 0.08f * (float)(sh->pd.n1 + 2 * sh->pd.n2)) * kWalkClock;
@@ -1100,7 +1101,9 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
     if (lane == 0) {
       sh->cells = sh->cells64 = 0ull;
       if (rc == WALK_GIVE_UP && leader)
-        st->walk_off |= phase == PH_SEARCH ? 1 << PH_SEARCH : 1 << PH_DFD | 1 << PH_VEFD;
+        st->walk_off |= phase == PH_SEARCH                 ? 1 << PH_SEARCH
+                        : phase == PH_DFD && st->walk_ve > 0.0 ? 1 << PH_DFD  // (the VE-FD is at hand)
+                                                               : 1 << PH_DFD | 1 << PH_VEFD;
       if (leader && band) st->walk_band = 1;
     }
     if (rc == WALK_ERROR || !walk_barrier(wa, g)) return false;
@@ -2971,13 +2974,21 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
           m |= 1u << hs[p].phase;
       return m;
     };
-    auto pass = [&](int parts, bool walk_search) -> int {
+    // parts of the strips in order, then the search's walk; a VE-FD that a walk has found ahead of a
+    // DFD that it gave up is taken, not swept again
+    auto pass = [&](int parts, bool walk_search, bool take_ve) -> int {
       RFD_CUDA(cudaMemsetAsync(dbase + L.zero_begin, 0, L.zero_end - L.zero_begin, st));
+      nwalk = 0;
+      if (take_ve) {
+        int rc2 = strips(1);
+        if (!rc2) rc2 = walk(2);
+        if (rc2) return rc2;
+        parts &= ~1;
+      }
       int rc2 = strips(parts);
       if (rc2) return rc2;
       if (walk_search) {
         if (ctx->timing) RFD_CUDA(record(2));
-        nwalk = 0;
         rc2 = walk(4);
         if (rc2) return rc2;
         if (ctx->timing) RFD_CUDA(record(3));
@@ -2991,11 +3002,13 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     const unsigned o1 = open(false);
     if (o1 & before) {
       const bool ws = mode == MODE_DISTANCE && (open(true) & before) != 0;
-      const int rc2 = pass((int)(o1 >> PH_DFD & 1) | 2 | (ws ? 0 : 4), ws);
+      bool ve = false;
+      for (int64_t p = 0; p < npairs; ++p) ve = ve || (hs[p].phase == PH_DFD && hs[p].walk_ve > 0.0);
+      const int rc2 = pass((int)(o1 >> PH_DFD & 1) | 2 | (ws ? 0 : 4), ws, ve);
       if (rc2) return rc2;
     }
     if (hmisc[1] == 0 && open(false)) {
-      const int rc2 = pass(4, false);
+      const int rc2 = pass(4, false, false);
       if (rc2) return rc2;
     }
   }

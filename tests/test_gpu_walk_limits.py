@@ -103,3 +103,15 @@ def test_thin_pairs_run_on_the_strips_at_once(ctx, strips, built):
         count.append(c.phase_times()["launches"])
         c.phase_times(0)
     assert count[:3] == count[3:]
+
+
+def test_vefd_ahead_of_a_given_up_dfd_is_kept(ctx, strips, built):
+    """A group sweeps the VE-FD before the DFD; where it then gives the DFD up (a stretch of this pair
+    is wide) the strips sweep the DFD only."""
+    P, Q = built.gen_pair(1, 2, 60000, 45001, 100.0, 0.1, 970302523, 1)
+    ms = []
+    for c in (ctx, strips):
+        c.phase_times(1)
+        ms.append((c.bounds(P, Q, quirks=False), c.phase_times(0)["vefd_ms"]))
+    assert ms[0][0] == ms[1][0]
+    assert ms[0][1] < 0.3 * ms[1][1]
