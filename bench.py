@@ -44,17 +44,18 @@ WORKLOAD = ("long pair: 2 x 200,000-point 3D spline paths (2,000 waypoints U[-10
             "20-knot time warp, noise 0.1, seed 1); FD to 2^-33 relative")
 # algorithmic FP64 flops per cell (fma = 2, sqrt/div = 1), from the reference expressions:
 # DFD .cu:615-626, VE-FD .cu:373-419, decision .cu:1173-1244
-# ncu dram__bytes_read.sum + dram__bytes_write.sum on the 20,000-point case: one decision
-# round, both halves of the split pair (mirror 3.584768 MB + forward 4.161792 MB); one VE-FD
-# launch of the unsplit pair (two launches averaged; the split VE-FD was not captured)
-DEC_DRAM_BYTES_20K = 3.584768e6 + 4.161792e6
-VEFD_DRAM_BYTES_20K = 4.31e6
+# ncu dram__bytes.sum per launch on the 20,000-point case, learned form: one decision and the
+# VE-FD (walk_kernel), the inflated coarse sweep (dfd_fed_kernel<true>)
+DEC_DRAM_BYTES_20K = 2.98e6
+VEFD_DRAM_BYTES_20K = 3.07e6
+COARSE_DRAM_BYTES_20K = 0.60e6
 COARSE_UB = 6  # the learned form's upper bound: inflated DFD of every 6th point (rfd.h coarse_ub)
 ARITY = 4  # batched forms: radii per round for the longest-chain pairs (rfd.h search_arity)
 DFD_DRAM_BYTES_200K = 31.5e6 + 68.4e6  # ncu, the exact DFD launch of the long pair (32-row ring)
-KERNEL_OF_PHASE = {"dfd": f"dfd_kernel<{'1, INFL' if COARSE_UB else '8'}>",
-                   "vefd": "team_kernel<K_VEFD> (forward and mirror halves)",
-                   "search": "team_kernel<K_DEC> (forward and mirror halves)"}
+# (the walk may give a phase up; the strips' kernels then finish it)
+KERNEL_OF_PHASE = {"dfd": "dfd_fed_kernel<true>" if COARSE_UB else "walk_kernel (DFD)",
+                   "vefd": "walk_kernel (VE-FD)",
+                   "search": "walk_kernel (decision)"}
 FLOPS_PER_CELL = {"dfd": lambda d: 3 * d + 3 + (4 if COARSE_UB else 0),  # + sqrt, 2 adds, square
                   "vefd": lambda d: 24 * d + 2,
                   "search": lambda d: 12 * d + 22}
@@ -639,12 +640,14 @@ def main():
     achieved = flops / (ph_ms[dom] * 1e-3) / 1e12
     traffic = None
     if dom in ("search", "vefd"):
-        # ncu dram__bytes_read.sum + dram__bytes_write.sum of one decision (VE-FD) launch on the
-        # 20,000-point case (cold cache: every touched point record and boundary word once);
-        # the touched data grows with the points, not the cells, so it scales by n1 + n2
+        # one decision (VE-FD) launch on the 20,000-point case (cold cache: every touched point
+        # and record once); the touched data grows with the points, not the cells, so it scales
+        # by n1 + n2
         per20k = DEC_DRAM_BYTES_20K if dom == "search" else VEFD_DRAM_BYTES_20K
         traffic = per20k * (n1 + n2) / 40000
-    elif dom == "dfd" and not COARSE_UB:
+    elif dom == "dfd" and COARSE_UB:
+        traffic = COARSE_DRAM_BYTES_20K * (n1 + n2) / 40000
+    elif dom == "dfd":
         # ncu dram__bytes_read.sum + dram__bytes_write.sum of the DFD launch on the full
         # 200,000-point pair (one pass): curves and the ring rows L2 evicts, scaled by points
         traffic = DFD_DRAM_BYTES_200K * (n1 + n2) / 400000
@@ -693,12 +696,9 @@ def main():
                      "peak_source": "measured FP64 FMA throughput (rfd_fp64_peak), this GPU",
                      "flops_per_cell": FLOPS_PER_CELL[dom](d), "cells": cells[dom],
                      "traffic_note": ("bytes per launch, ncu capture of the full-size launch"
-                                      if dom == "dfd" else
-                                      "bytes per probe round (both halves of the split pair), "
-                                      "ncu cold-cache capture at 20k points scaled by points"
-                                      if dom == "search" else
-                                      "bytes of one unsplit VE-FD launch, ncu cold-cache capture "
-                                      "at 20k points scaled by points")},
+                                      if dom == "dfd" and not COARSE_UB else
+                                      "bytes per launch, ncu cold-cache capture at 20k points "
+                                      "scaled by points")},
         # the pruned sweeps are bound by their dependency chain, not by flops or bytes: the
         # wavefront has n1 + n2 anti-diagonals, so this is the latency each one adds
         "critical_path": {
