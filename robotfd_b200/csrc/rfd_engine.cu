@@ -648,10 +648,13 @@ __device__ void tree_done(const WaveArgs& wa, PairState* g) {
 // Sets up pair g's next probe (phase PH_SEARCH, split set by next_probe): a k-ary round's
 // members get their radii and states; returns the decisions of the round (1: one decision at
 // the split).  Queues nothing: a launch round takes the members' strips from its item list,
-// the continuous search queues them (start_next).  One thread.
+// the continuous search queues them (start_next).  One thread.  TREE: rounds of the next probes
+// (a kernel of their own: their code in the plain one cost its sweep registers, 36 bytes of spills
+// and a tenth of a dense search).
+template <bool TREE>
 __device__ int kary_arm(const WaveArgs& wa, PairState* g, int S) {
+  if constexpr (TREE) return g->kary_cap > 0 ? tree_arm(wa, g, S) : 1;
   int n = 1;
-  if (wa.kary_tree) return g->kary_cap > 0 ? tree_arm(wa, g, S) : 1;
   if (g->kary_cap > 0 && wa.kary_k >= 2 && g->srch.mode == SM_BISECT &&
       ld_volatile(wa.active_pairs) <= wa.kary_gate) {
     // the widest round whose decisions still close the gap within the probe cap: halvings
@@ -691,6 +694,7 @@ __device__ int kary_arm(const WaveArgs& wa, PairState* g, int S) {
 }
 
 // Continuous search: queues the first strips of every decision of pair p's armed probe.
+template <bool TREE>
 __device__ void start_armed(const WaveArgs& wa, PairState* g, int p, int S) {
   if (g->kary_n < 2) {
     start_probe(wa, g, p, S);
@@ -698,25 +702,28 @@ __device__ void start_armed(const WaveArgs& wa, PairState* g, int p, int S) {
   }
   const int n = g->kary_n;
   for (int k = 0; k < n; ++k)
-    if (k == 0 || kary_member(wa, g, k)->kary_in) start_probe(wa, kary_member(wa, g, k), k == 0 ? p : g->kary_base + (k - 1), S);
+    if (!TREE || k == 0 || kary_member(wa, g, k)->kary_in)
+      start_probe(wa, kary_member(wa, g, k), k == 0 ? p : g->kary_base + (k - 1), S);
 }
 
 // Continuous search: arms and starts pair p's next probe.  One thread.
+template <bool TREE>
 __device__ void start_next(const WaveArgs& wa, PairState* g, int p, int S) {
-  kary_arm(wa, g, S);
-  start_armed(wa, g, p, S);
+  kary_arm<TREE>(wa, g, S);
+  start_armed<TREE>(wa, g, p, S);
 }
 
 // A decision of a k-ary round ended (in the continuous search, its boundary words are cleared);
 // the round's last one combines the outcomes and arms the pair's next probe, and in the
 // continuous search (queue) starts it.  One thread.
+template <bool TREE>
 __device__ void kary_done(const WaveArgs& wa, PairState* ms, int S, bool queue) {
   const int p = ms->kary_real;
   PairState* g = wa.st + p;
   __threadfence();
   if (atomicSub(&g->kary_left, 1) != 1) return;
   __threadfence();
-  if (wa.kary_tree) {
+  if constexpr (TREE) {
     tree_done(wa, g);
   } else {
     const int n = g->kary_n;
@@ -743,8 +750,8 @@ __device__ void kary_done(const WaveArgs& wa, PairState* ms, int S, bool queue) 
   g->kary_n = 0;
   next_probe(g, wa.active_pairs);
   if (g->phase == PH_SEARCH && g->active) {
-    if (queue) start_next(wa, g, p, S);
-    else kary_arm(wa, g, S);
+    if (queue) start_next<TREE>(wa, g, p, S);
+    else kary_arm<TREE>(wa, g, S);
   }
 }
 
@@ -754,8 +761,12 @@ __global__ void search_queue_init_kernel(const PairDesc* pairs, PairState* st, i
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npairs; p += gridDim.x * blockDim.x) {
     if (st[p].phase != PH_SEARCH || !st[p].active) continue;
     const int S = (pairs[p].n1 - 1 + 31) >> 5;
-    if (wa.kary_tree && st[p].kary_cap > 0) kary_arm(wa, st + p, S);
-    start_armed(wa, st + p, p, S);
+    if (wa.kary_tree) {
+      if (st[p].kary_cap > 0) kary_arm<true>(wa, st + p, S);
+      start_armed<true>(wa, st + p, p, S);
+    } else {
+      start_armed<false>(wa, st + p, p, S);
+    }
   }
 }
 
@@ -773,7 +784,7 @@ __global__ void search_queue_init_kernel(const PairDesc* pairs, PairState* st, i
 // MIR: the mirror halves of split pairs (meet in the middle), a kernel of their own so that
 // the forward kernel's registers stay as they are; it runs beside the forward kernel, on
 // another stream, each on half the teams.
-template <int KIND, int NW = kTeamThreads / 32, bool MIR = false>
+template <int KIND, int NW = kTeamThreads / 32, bool MIR = false, bool TREE = false>
 __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) team_kernel(WaveArgs wa) {
   constexpr int H = NW - 1;  // helper warps
   extern __shared__ __align__(128) unsigned char team_smem[];
@@ -857,22 +868,24 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) team_kernel(WaveArgs
         const int n = atomicAdd(&st->done_count, 1);
         // (the halves of a split pair, split != 0, end in split_meet_kernel instead; read
         // from the descriptor here, not kept in registers across the strip)
-        if (n == S - 1 && !MIR && !ld_volatile(&wa.pairs[p].split)) {
-          __threadfence();
-          finalize<KIND>(st, pd, wa.active_pairs);
-          __threadfence();
-          if (dyn && st->phase == PH_SEARCH && st->active) sh->push = 1;
-          else if (dyn && st->phase == PH_KWAIT) sh->push = 2;
-          // launch rounds: the next launch runs what is armed here (its fill resets the rows)
-          else if (KIND == K_DEC && !dyn && st->phase == PH_KWAIT) kary_done(wa, st, S, false);
-          else if (KIND == K_DEC && !dyn && st->phase == PH_SEARCH && st->active &&
-                   st->kary_cap > 0 && !wa.kary_tree)
-            kary_arm(wa, st, S);
+        if constexpr (!MIR) {
+          if (n == S - 1 && !ld_volatile(&wa.pairs[p].split)) {
+            __threadfence();
+            finalize<KIND>(st, pd, wa.active_pairs);
+            __threadfence();
+            if (dyn && st->phase == PH_SEARCH && st->active) sh->push = 1;
+            else if (dyn && st->phase == PH_KWAIT) sh->push = 2;
+            // launch rounds: the next launch runs what is armed here (its fill resets the rows)
+            else if (KIND == K_DEC && !dyn && st->phase == PH_KWAIT) kary_done<TREE>(wa, st, S, false);
+            else if (KIND == K_DEC && !dyn && st->phase == PH_SEARCH && st->active &&
+                     st->kary_cap > 0 && !wa.kary_tree)
+              kary_arm<TREE>(wa, st, S);
+          }
         }
       }
     }
     __syncthreads();
-    if (KIND == K_DEC && sh->push) {
+    if (KIND == K_DEC && !MIR && sh->push) {
       // the probe's written boundary words back to "not yet written", one strip per warp
       const long long C = pd.n2 - 1;
       for (int r = warp; r < S - 1; r += NW) {
@@ -885,8 +898,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) team_kernel(WaveArgs
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) {
-        if (sh->push == 1) start_next(wa, st, p, S);
-        else kary_done(wa, st, S, true);
+        if (sh->push == 1) start_next<TREE>(wa, st, p, S);
+        else kary_done<TREE>(wa, st, S, true);
       }
     }
   }
@@ -1531,14 +1544,14 @@ dim3 prep_grid(int64_t longest, int64_t npairs) {
 }
 
 // The team kernel of the context's shape (warps per team) on its grid (grid > 0: that many
-// teams); MIR: the mirror kernel of split pairs.
-template <int KIND, bool MIR = false>
+// teams); MIR: the mirror kernel of split pairs; TREE: with tree rounds.
+template <int KIND, bool MIR = false, bool TREE = false>
 void launch_team(const rfd_context* ctx, const WaveArgs& wa, cudaStream_t st, int grid = 0) {
   const int g = grid > 0 ? grid : ctx->team_grid[KIND];
   if (ctx->team_warps == 4)
-    team_kernel<KIND, 4, MIR><<<g, 128, team_smem_bytes<KIND>(), st>>>(wa);
+    team_kernel<KIND, 4, MIR, TREE><<<g, 128, team_smem_bytes<KIND>(), st>>>(wa);
   else
-    team_kernel<KIND, 8, MIR><<<g, 256, team_smem_bytes<KIND>(), st>>>(wa);
+    team_kernel<KIND, 8, MIR, TREE><<<g, 256, team_smem_bytes<KIND>(), st>>>(wa);
 }
 
 // Row of rfd_context::team_grids for a team shape.
@@ -2812,7 +2825,8 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
       }
       search_queue_init_kernel<<<(int)std::min<int64_t>((npairs + 255) / 256, 1024), 256, 0, st>>>(
           dt, ds, (int)npairs, wa);
-      launch_team<K_DEC>(ctx, wa, st);
+      if (ktree) launch_team<K_DEC, false, true>(ctx, wa, st);
+      else launch_team<K_DEC>(ctx, wa, st);
       RFD_CUDA(cudaGetLastError());
       launches += 2;
       wa.nitems = nstatic;
@@ -3217,6 +3231,10 @@ int32_t rfd_context_create(int32_t device, rfd_context** out) {
         cudaFuncSetAttribute(team_kernel<K_VEFD, 4, true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ve) != cudaSuccess ||
         cudaFuncSetAttribute(team_kernel<K_DEC, 4, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_dec) != cudaSuccess ||
+        cudaFuncSetAttribute(team_kernel<K_DEC, 8, false, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_dec) != cudaSuccess ||
+        cudaFuncSetAttribute(team_kernel<K_DEC, 4, false, true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_dec) != cudaSuccess) {
       delete c;
       return fail(RFD_ERR_CUDA, "cudaFuncSetAttribute(team smem)");
