@@ -204,7 +204,8 @@ int32_t rfd_distance_batch(rfd_context* ctx, int64_t npairs, const double* const
 /* Autotuner of the DFD sweep (no reference counterpart: the reference fixes its launch shape,
    src/intersection_algorithm_in_parallel.cu:1268-1326).  Times rows per lane (1, 2, 4, 8: the
    strip height) and the row layout (0 stacked, 1 skewed) on the caller's pairs, `reps` timed
-   sweeps each after one untimed one, and keeps the fastest in the context for later calls.
+   sweeps each after one untimed one, and keeps the fastest in the context for later calls.  The
+   timed calls run on the strips that the shapes apply to: no walk sweeps, no fed strips.
    ms_out (optional): 8 doubles, ms per sweep at [rows index * 2 + layout].  best_out
    (optional): 2 ints, the rows and layout kept.  Curves as rfd_distance_batch (opt->memory). */
 int32_t rfd_autotune(rfd_context* ctx, int64_t npairs, const double* const* c1s, const int64_t* n1s,
@@ -216,8 +217,8 @@ int32_t rfd_autotune(rfd_context* ctx, int64_t npairs, const double* const* c1s,
    team (4 or 8), the switch point from probe rounds run as launches to the continuous queue
    (a quarter of the team count of active pairs, the team count, or the queue from the first
    probe: INT32_MAX) and the continuous search's start window (1, 2 or 4
-   strips), on whole solves of the caller's pairs with the caller's options (`reps` timed calls
-   each, after one untimed one), and keeps the fastest in the context for later calls.
+   strips), on whole solves of the caller's pairs with the caller's options, without walk sweeps
+   (`reps` timed calls each, after one untimed one), and keeps the fastest in the context for later calls.
    ms_out (optional): 18 doubles, ms per solve at [(warps index * 3 + switch index) * 3 +
    window index].  best_out (optional): 3 ints, warps per team, switch point, window kept.
    The strip height is the warp width (32 rows, a lane per row) and is not tuned. */

@@ -44,9 +44,10 @@
 //
 // What bounds it: the chain of a band's blocks.  A decision's block takes about 5,300 cycles (the
 // rows 2,900, waiting for the tile 900, the next block's choice 500; a tile is ready 3,500 after
-// its request), a VE-FD or DFD block with values about 10,000.  Against the strips, one pair:
-// search of 20,000 x 19,000 points 155 ms and 4.6 (37 probes), 2,000 x 1,900 17 and 2.7; bounds of
-// 60,000 x 45,000 points 35 and 1.8; VE-FD and one decision of 200,000 x 200,000 90 and 7.0.
+// its request), a VE-FD or DFD block with values about 10,000.  Against the strips, medians over
+// twelve pairs of a size: search of 20,000 x 19,000 points 180 ms and 7.8 (4.2 to 16.7), 2,000 x 1,900
+// 18.5 and 3.5; VE-FD and one decision of 200,000 x 200,000 95 and 3.8; bounds of 60,000 x 45,000
+// points 35 and 2.2 to 5.2 where the walk holds, 27 to 32 where it gives the DFD up.
 #pragma once
 
 #include "rfd_device.cuh"
