@@ -805,8 +805,10 @@ __device__ __forceinline__ void walk_values(const WalkShared* sh, int slot, int 
   __syncwarp();
   omask = __ballot_sync(kFull, (bot < dead) & (lane < nr));
   if (lane < nr) bout[lane] = bot;
+  // (a sweep that ended before lane 31 came to the last column, all dead from there on, leaves it
+  // what it handed up from an earlier column; the other lanes' live values keep the sweep going)
   y = bot;
-  f = carry;
+  f = t - lane >= nc ? carry : dead;
   __syncwarp();
 }
 

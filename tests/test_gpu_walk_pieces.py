@@ -72,3 +72,21 @@ def test_last_pairs_of_a_batch_of_like_pairs(strips, built):
                 assert [[x[k] for k in KEYS] for x in a] == [[x[k] for k in KEYS] for x in w]
     finally:
         c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,m", [(33, 32), (65, 45), (97, 57), (161, 21), (577, 27), (33, 12)])
+def test_vefd_of_whole_last_block_rows(ctx, strips, built, n, m):
+    """The last block row has 32 rows and the level grows past dead sweeps: what the last row last
+    handed up is not the last cell's value unless the sweep came that far."""
+    for seed in range(60):
+        g = np.random.default_rng(1000 * n + seed)
+        d = 2 + seed % 2
+        if seed % 3:
+            P, Q = np.cumsum(g.standard_normal((n, d)), 0), np.cumsum(g.standard_normal((m, d)), 0)
+        else:
+            t, u = 2 * np.pi * np.linspace(0, 3, n), 2 * np.pi * np.linspace(0, 3, m)
+            P, Q = (np.stack([np.cos(v), np.sin(v)] + [0.1 * v] * (d - 2), 1) +
+                    0.2 * g.standard_normal((len(v), d)) for v in (t, u))
+        assert ctx.bounds(P, Q, quirks=False) == strips.bounds(P, Q, quirks=False)
+        assert ctx.bounds(Q, P, quirks=False) == strips.bounds(Q, P, quirks=False)
