@@ -44,7 +44,7 @@ def test_a_tuned_context_keeps_the_fed_strips(built):
             if tune:
                 c.autotune([R], [S], reps=1)
             best = 1e9
-            for _ in range(6):
+            for _ in range(20):
                 c.phase_times(1)
                 c.distance(P, Q, precise=True, coarse_ub=6, max_probes=1)
                 best = min(best, c.phase_times(0)["dfd_ms"])

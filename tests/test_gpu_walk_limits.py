@@ -70,23 +70,29 @@ def test_routes_agree_in_calls_of_several(ctx, strips, built, kind, kw):
         assert [[x[k] for k in KEYS] for x in a] == [[x[k] for k in KEYS] for x in b]
 
 
-def best(f, reps=20):
-    f()
-    t = []
-    for _ in range(reps):
-        t0 = time.perf_counter()
-        f()
-        t.append(time.perf_counter() - t0)
-    return min(t)
+def least(f, g, reps=40):
+    """Least times of two calls, taken in turn."""
+    t = [[], []]
+    for _ in range(reps + 1):
+        for k, h in enumerate((f, g)):
+            t0 = time.perf_counter()
+            h()
+            t[k].append(time.perf_counter() - t0)
+    return min(t[0][1:]), min(t[1][1:])
 
 
 @pytest.mark.parametrize("kind,n1,n2", [("indep", 300, 260), ("indep", 600, 610), ("noise", 600, 610),
                                         ("loops", 1281, 1100)])
 def test_wide_bands_cost_little_more_than_the_strips(ctx, strips, built, kind, n1, n2):
-    """Before the walk kept to a share of the strips' time: 5, 11, 8 and 15 times as long."""
+    """Before the walk kept to a share of the strips' time: 5, 11, 8 and 15 times as long.  (Other
+    users of the host can disturb calls for a second or two: up to four tries.)"""
     P, Q = curves(built, kind, 2, n1, n2)
-    assert best(lambda: ctx.bounds(P, Q, quirks=False)) < \
-        2.5 * best(lambda: strips.bounds(P, Q, quirks=False))
+    for _ in range(4):
+        a, b = least(lambda: ctx.bounds(P, Q, quirks=False), lambda: strips.bounds(P, Q, quirks=False))
+        if a < 2.5 * b:
+            return
+        time.sleep(1.0)
+    assert a < 2.5 * b
 
 
 def test_thin_pairs_run_on_the_strips_at_once(ctx, strips, built):
@@ -109,9 +115,14 @@ def test_vefd_ahead_of_a_given_up_dfd_is_kept(ctx, strips, built):
     """A group sweeps the VE-FD before the DFD; where it then gives the DFD up (a stretch of this pair
     is wide) the strips sweep the DFD only."""
     P, Q = built.gen_pair(1, 2, 60000, 45001, 100.0, 0.1, 970302523, 1)
-    ms = []
+    ms, got = [], []
     for c in (ctx, strips):
         c.phase_times(1)
-        ms.append((c.bounds(P, Q, quirks=False), c.phase_times(0)["vefd_ms"]))
-    assert ms[0][0] == ms[1][0]
-    assert ms[0][1] < 0.3 * ms[1][1]
+        t = []
+        for _ in range(6):
+            got.append(c.bounds(P, Q, quirks=False))
+            t.append(c.phase_times(1)["vefd_ms"])
+        c.phase_times(0)
+        ms.append(min(t))
+    assert len(set(got)) == 1
+    assert ms[0] < 0.3 * ms[1]
