@@ -995,7 +995,7 @@ __device__ bool walk_pair(const WaveArgs& wa, const WalkArgs& ka, WalkShared* sh
   const float S = (float)(in.n1 + 30) / 32.f, K = (float)(in.n2 + 30) / 32.f;
   const float worth =
       npairs > 1 ? fmaxf(1.f, 0.5f * (float)min(npairs, ka.teams) * S / (float)ka.teams) : 1.f;
-  const float strips_seg = worth * (20.f + 7.5f * S + 3.5f * K) * kWalkClock;
+  const float strips_seg = worth * (10.f + 7.5f * S + 3.5f * K) * kWalkClock;
   const float strips_dfd =
       worth * (20.f + 0.08f * (float)(sh->pd.n1 + 2 * sh->pd.n2)) * kWalkClock;
   // A phase begins: the share of the strips' time, and so many us more, that all its sweeps may take,
@@ -1144,7 +1144,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) walk_kernel(WaveArgs wa, Walk
     return;
   }
   const int lane = threadIdx.x;
-  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, 0, -1, WalkCut{0, 0, 0}, 0, -1, WALK_BY_TIME, 0, 0.f, 0.f, false, 0u,
+  Walk w{0u, 0u, -1, -1, 0, 0, 0, 0, 0, 0, -1, WalkCut{0, 0, 0}, 0, -1, WALK_BY_TIME, 0, 0.f, 0.f, false, 0u,
          ka.stop + group};
   WalkGroup g;
   g.size = size;
@@ -1890,12 +1890,12 @@ int run_batch(rfd_context* ctx, int64_t npairs, const double* const* c1s, const 
     return walks && hi >= kWalkAspectFrom && hi >= kWalkAspect * lo;
   };
   // Phases of a pair (bit 1 << phase) that the walk leaves to the strips from the start: all of a thin
-  // pair's, and a lone decision on a grid of up to three pieces (600 x 610 points: 0.36 ms on the
-  // strips, 0.23 to 0.28 walked where the band is thin, 0.55 where it is not).
+  // pair's, and a lone decision on a grid of one piece (300 x 260 points: 0.25 ms on the strips, a
+  // walk saves a seventh of that at most and costs half as much again where the band is wide).
   auto walk_blocks = [&](int64_t p) { return (n1s[p] + 30) / 32 + (n2s[p] + 30) / 32; };
   auto walk_off = [&](int64_t p) -> int {
     if (thin(p)) return 1 << PH_DFD | 1 << PH_VEFD | 1 << PH_SEARCH;
-    return mode == MODE_DECIDE && walk_blocks(p) < 4 * kWalkStretch ? 1 << PH_SEARCH : 0;
+    return mode == MODE_DECIDE && walk_blocks(p) < 2 * kWalkStretch ? 1 << PH_SEARCH : 0;
   };
   auto tree_fits = [&](int64_t p) {
     return thin(p) && n1s[p] >= 2 && n2s[p] >= 2 && (trows(p) - 1 + 31) / 32 * 3 <= ctx->team_grid[K_DEC] * 5 / 4;
@@ -3954,13 +3954,8 @@ extern "C" int32_t rfd_decide_noalloc(const double* c1, int64_t n1, const double
   ka.phases = 4;
   ka.quota = 1;
   ka.teams = nd.team_grid;
-  // (no walk on grids below kWalkLeast blocks, rows and columns together: 150 x 140 points take 100 us
-  // on the strips, 75 to 100 with the walk, 200 where the band is wide)
-  constexpr int64_t kWalkLeast = 16;
-  if ((n1 + 30) / 32 + (n2 + 30) / 32 >= kWalkLeast) {
-    walk_kernel<<<1, kWalkThreads, kWalkSmem, st>>>(wa, ka);
-    RFD_CUDA(cudaGetLastError());
-  }
+  walk_kernel<<<1, kWalkThreads, kWalkSmem, st>>>(wa, ka);
+  RFD_CUDA(cudaGetLastError());
   bnd_fill_kernel<<<dim3(256, 1), 256, 0, st>>>(ddesc, dstate, 1, PH_SEARCH, nullptr, nullptr, 0, 0);
   RFD_CUDA(cudaGetLastError());
   team_kernel<K_DEC, 8><<<nd.team_grid, kTeamThreads, team_smem_bytes<K_DEC>(), st>>>(wa);

@@ -45,9 +45,9 @@
 // What bounds it: the chain of a band's blocks.  A decision's block takes about 5,300 cycles (the
 // rows 2,900, waiting for the tile 900, the next block's choice 500; a tile is ready 3,500 after
 // its request), a VE-FD or DFD block with values about 10,000.  Against the strips, medians over
-// twelve pairs of a size: search of 20,000 x 19,000 points 180 ms and 7.8 (4.2 to 16.7), 2,000 x 1,900
+// twelve pairs of a size: search of 20,000 x 19,000 points 180 ms and 7.7 (4.1 to 16.3), 2,000 x 1,900
 // 18.5 and 3.5; VE-FD and one decision of 200,000 x 200,000 95 and 3.8; bounds of 60,000 x 45,000
-// points 35 and 2.2 to 5.2 where the walk holds, 27 to 32 where it gives the DFD up.
+// points 35 and 2.1 to 5.0 where the walk holds, 26 to 32 where it gives the DFD up.
 #pragma once
 
 #include "rfd_device.cuh"
@@ -818,7 +818,7 @@ struct Walk {
   int pi, pj;             // the outstanding request (pi < 0: none)
   int cur, n;             // list of the row below: buffer and live chunks
   long long t0;           // cycle the running walk began
-  int blocks;             // its blocks and listed edges (256 count as a block)
+  int blocks, effort;     // its blocks, and with their listed edges (256 count as a block)
   int rec_from, rec_end;  // block rows whose records this sweep can be met at
   // where an earlier sweep's band ran: this member's piece, cut so that pieces take equal
   // stretches of the band, and the chunks it entered it in (lo > hi: not known)
@@ -847,26 +847,34 @@ enum WalkMode : int { WALK_ALONE = 0, WALK_RECORD = 1, WALK_AGAIN = 2 };
 //                   lists a few hundred edges a block and goes from block to block right or up (a
 //                   pair of many, each walked by one CTA: the strips' time is the call's then);
 //   WALK_BY_REST    a lone CTA's walk, once a twelfth of the strips' time has passed (60 us at
-//                   most): if the rest at this rate takes longer than the strips (what is spent is
-//                   spent; 1.15: rates vary along a band);
+//                   most): if the rest takes longer than the strips (what is spent is spent; 1.15:
+//                   rates vary along a band).  The rest is the blocks still ahead at the rate so
+//                   far, or the rows still to come with as many chunks as the list has now;
 //   WALK_BY_TIME    a group's: the phase's deadline; and a piece, where `pace` says so, against a thin
 //                   band's rate, which is about 5 us a block row or column for the decision and 8
-//                   for the others.  A wide band's blocks cost 16 us and more (all of their edges
-//                   listed), and nothing says that before they are walked.
+//                   for the others.  A wide band's blocks cost 4 to 16 us each (most of their edges
+//                   listed), a row of them tells (150 x 140 unrelated points, decide_noalloc: 205
+//                   us walked, 100 on the strips, 130 given up).
 enum WalkRule : int { WALK_BY_EFFORT = 0, WALK_BY_REST, WALK_BY_TIME };
-__device__ __forceinline__ bool walk_slow(const Walk& w, int ahead, int total) {
-  if (w.rule == WALK_BY_EFFORT) return w.blocks > 64 + 4LL * (ahead - 1);
+// ahead, total: blocks come ahead, of the grid's rows and columns; chunks: of the list; rows, left: the
+// piece's, and those still to come.  Asked every fourth block (the code that runs once a block is
+// fetched anew: asked every block it took 7 % of a decision).
+__device__ __forceinline__ bool walk_slow(const Walk& w, int ahead, int total, int chunks, int rows,
+                                          int left) {
+  if (w.rule == WALK_BY_EFFORT) return w.effort > 64 + 4LL * (ahead - 1);
   constexpr float us = kWalkClock;
   const long long now = clock64();
-  const float spent = (float)(now - w.t0);
-  bool slow;
+  const float spent = (float)(now - w.t0), blocks = (float)w.blocks;
+  const float to_come = spent * (float)(chunks * left);  // (times the blocks)
   if (w.rule == WALK_BY_REST)
-    slow = spent > fminf(w.strips / 12.f, 60.f * us) &&
-           spent * (float)(total - ahead) > 1.15f * w.strips * (float)ahead;
-  else
-    slow = now > w.deadline ||
-           (w.pace > 0.f && spent > fmaxf(15.f * us + w.pace * (float)ahead, 0.12f * w.strips));
-  return bcast((int)slow) != 0;
+    return spent > fminf(w.strips / 12.f, 60.f * us) &&
+           (spent * (float)(total - ahead) > 1.15f * w.strips * (float)ahead ||
+            to_come > 1.15f * w.strips * blocks);
+  if (now > w.deadline) return true;
+  if (!(w.pace > 0.f)) return false;
+  const float may = fmaxf(15.f * us + w.pace * (float)ahead, 0.12f * w.strips);
+  const float may_all = fmaxf(15.f * us + w.pace * (float)(2 * rows), 0.12f * w.strips);
+  return spent > may || (spent > 10.f * us && to_come > (1.5f * may_all - spent) * blocks);
 }
 // Tells the other members that this sweep's end is known, or that it is given up.
 __device__ __forceinline__ void walk_stop(const Walk& w) {
@@ -984,19 +992,25 @@ __device__ int walk_rows(const WaveArgs& wa, WalkShared* sh, Walk& w, int i0, in
       unsigned V = __ballot_sync(kFull, walk_live<KIND>(F));
       k += have;
       // (on its way while the tile is waited for)
-      const unsigned stop = mode != WALK_ALONE ? *(volatile unsigned*)w.stop : 0u;
+      const bool ask = (w.blocks & 3) == 3;
+      const unsigned stop = ask && mode != WALK_ALONE ? *(volatile unsigned*)w.stop : 0u;
       const int slot = walk_get(wa, sh, w, i, j);
       if (slot < 0) { status = WALK_ERROR; break; }
       j_min = min(j_min, j);
       j_max = max(j_max, j);
-      w.blocks += 1 + (sh->cnt[slot] >> 8);
-      if (mode != WALK_ALONE && bcast(stop) == w.sweeps) {
-        status = WALK_STOPPED;
-        break;
-      }
-      if (walk_slow(w, (i - i0) + (j_max - j_min) + 1, nbr + nbc) || (on == kWalkCap && !loose)) {
+      w.blocks += 1;
+      w.effort += 1 + (sh->cnt[slot] >> 8);
+      if (on == kWalkCap && !loose) {
         status = WALK_GIVE_UP;
         break;
+      }
+      if (ask) {
+        const int quit =
+            mode != WALK_ALONE && stop == w.sweeps ? WALK_STOPPED
+            : walk_slow(w, (i - i0) + (j_max - j_min) + 1, nbr + nbc, max(on, w.n), i1 - i0, i1 - 1 - i)
+                ? WALK_GIVE_UP : WALK_OK;
+        status = bcast(quit);
+        if (status != WALK_OK) break;
       }
       {
         // the next block: right when this one's last column has a live edge, else the next
@@ -1289,7 +1303,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
   w.cur = 0;
   w.n = 0;
   w.t0 = clock64();
-  w.blocks = 0;
+  w.blocks = w.effort = 0;
   w.rec_from = 0;
   w.rec_end = -1;
   double start = dead;
@@ -1453,7 +1467,7 @@ __device__ int walk_sweep(const WaveArgs& wa, WalkShared* sh, Walk& w, WalkGroup
     if (again) {
       walk_load_end(sh, w, g.end[from] + g.first + before);
       w.t0 = clock64();
-      w.blocks = 0;
+      w.blocks = w.effort = 0;
       c = 0.0;
       double r = none;
       int q = WALK_OK;
